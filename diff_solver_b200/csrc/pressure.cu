@@ -49,17 +49,48 @@ PressureWorkspace carve_pressure_workspace(void* base, const Grid& g) {
     };
     w.state = static_cast<SolverState*>(take(sizeof(SolverState)));
     w.partials = static_cast<double*>(take(sizeof(double) * kPartialSlots * kMaxPersistentBlocks));
+    w.slots = take(kSlotBytes);
     w.x64 = static_cast<double*>(take(sizeof(double) * n));
-    w.z = static_cast<float*>(take(sizeof(float) * n));
-    w.p0 = static_cast<float*>(take(sizeof(float) * n));
-    w.p1 = static_cast<float*>(take(sizeof(float) * n));
-    w.q = static_cast<float*>(take(sizeof(float) * n));
-    w.e = static_cast<float*>(take(sizeof(float) * n));
-    w.s = static_cast<float*>(take(sizeof(float) * n));
-    w.y = static_cast<float*>(take(sizeof(float) * n));
+    // sized for periodic axes, which pad most: the boundary modes come with the solve
+    const uint64_t padded = padded_cells(g, {2u, 2u, 2u, 2u, 2u, 2u});
+    const bool pad = padded <= padded_limit(n) && padded < (1ull << 31);
+    const size_t bytes = sizeof(float) * (pad ? padded : n);
+    w.z = static_cast<float*>(take(bytes));
+    w.p0 = static_cast<float*>(take(bytes));
+    w.p1 = static_cast<float*>(take(bytes));
+    w.q = static_cast<float*>(take(bytes));
+    w.e = static_cast<float*>(take(bytes));
+    w.s = static_cast<float*>(take(bytes));
+    w.y = static_cast<float*>(take(bytes));
+    if (pad) {
+        w.z1 = static_cast<float*>(take(bytes));
+        w.q1 = static_cast<float*>(take(bytes));
+        w.code = static_cast<uint8_t*>(take(padded));
+    }
+    w.padded = pad;
     w.bytes = off;
     return w;
 }
+
+namespace {
+
+struct PadExtents {
+    uint64_t pitch, rows, plane, total;
+};
+
+PadExtents pad_extents(const Grid& g, const uint32_t (&modes)[6]) {
+    auto wraps = [&](int d) { return modes[2 * d] == 2u && modes[2 * d + 1] == 2u; };
+    PadExtents e;
+    e.pitch = (static_cast<uint64_t>(g.nx) + (wraps(0) ? 2 : 1) + 3) / 4 * 4;
+    e.rows = static_cast<uint64_t>(g.ny) + (wraps(1) ? 2 : 1);
+    e.plane = e.pitch * e.rows;
+    e.total = e.plane * (static_cast<uint64_t>(g.nz) + 2) + 256;  // a warp's worth past the last plane
+    return e;
+}
+
+}  // namespace
+
+uint64_t padded_cells(const Grid& g, const uint32_t (&modes)[6]) { return pad_extents(g, modes).total; }
 
 size_t pressure_workspace_bytes(const Grid& g) { return carve_pressure_workspace(nullptr, g).bytes; }
 
@@ -947,6 +978,12 @@ __global__ void __launch_bounds__(kBlock, kSmooth ? 3 : 4) pcg_kernel(PcgArgs a)
     }
 }
 
+}  // namespace xs
+
+#include "pcg_single.cuh"
+
+namespace xs {
+
 // -------------------------------------------------- red-black Gauss-Seidel
 // operators.cu:885-902 applied to the cells of one parity.
 __device__ void rbgs_phase(const Operator& op, int parity, const float* rhs, float* p) {
@@ -1191,6 +1228,110 @@ unsigned fast_pass_blocks(const Grid& g) {
     return static_cast<unsigned>(std::min<uint64_t>((cell_count(g) / 4 + 255) / 256, 148 * 16));
 }
 
+PadGeom pad_geom(const Grid& g, const XsScalarBoundary& pb) {
+    const PadExtents e = pad_extents(g, pb.modes);
+    PadGeom p{};
+    p.nx = static_cast<uint32_t>(g.nx);
+    p.ny = static_cast<uint32_t>(g.ny);
+    p.nz = static_cast<uint32_t>(g.nz);
+    p.n = static_cast<uint32_t>(cell_count(g));
+    p.pitch = static_cast<uint32_t>(e.pitch);
+    p.rows = static_cast<uint32_t>(e.rows);
+    p.plane = static_cast<uint32_t>(e.plane);
+    p.base = p.plane;
+    p.total = static_cast<uint32_t>(e.total);
+    p.quads = (p.plane / 4u * p.nz + 31u) / 32u * 32u;
+    p.dnx = make_fastdiv(p.nx);
+    p.dny = make_fastdiv(p.ny);
+    p.dpitch = make_fastdiv(p.pitch);
+    p.drows = make_fastdiv(p.rows);
+    for (int d = 0; d < 3; ++d)
+        if (pb.modes[2 * d] == 2u && pb.modes[2 * d + 1] == 2u) p.periodic |= 1u << d;
+    return p;
+}
+
+// The single-synchronisation PCG, one CTA per SM.
+template <bool kSmooth, int kPer>
+XsStatus launch_cg(CgArgs& a, unsigned blocks, size_t smem, cudaStream_t stream) {
+    static DeviceOnce configured;
+    if (!configured.run([] { return cudaFuncSetAttribute(cg_kernel<kSmooth, kPer>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kCgMaxSmem)); }))
+        return XS_CUDA_ERROR;
+    if (cudaMemsetAsync(a.slots, 0, 2ull * blocks * kMaxSlotStride * sizeof(ulonglong2), stream) != cudaSuccess) return XS_CUDA_ERROR;
+    void* params[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(cg_kernel<kSmooth, kPer>), dim3(blocks), dim3(kCgThreads), params, smem, stream);
+    if (e != cudaSuccess) return check_cuda(e);
+    return check_launch();
+}
+
+// The brick of rows with the least surface for which `per` groups per thread
+// and one block per SM hold the grid and its surroundings; false: none.
+bool brick_for(const PadGeom& g, uint32_t resident, int per, bool smooth, BrickGeom& out, uint32_t& blocks) {
+    const uint64_t hold = static_cast<uint64_t>(per) * kCgThreads, width = (g.nx + 3ull) / 4ull;
+    uint64_t best = 0;
+    for (uint64_t by = 1; by <= g.ny && width * by <= hold; ++by) {
+        uint64_t bz = std::min<uint64_t>(g.nz, hold / (width * by));
+        const uint64_t slabs = (g.nz + bz - 1) / bz;
+        bz = (g.nz + slabs - 1) / slabs;  // as even as the same number of slabs allows
+        const uint64_t rows = (g.ny + by - 1) / by, around = 2 * width * (by + bz);
+        if (rows * slabs > resident || around > hold || (best != 0 && around * rows * slabs >= best)) continue;
+        if (brick_smem(static_cast<uint32_t>(width), static_cast<uint32_t>(by), static_cast<uint32_t>(bz), per, smooth) > kCgMaxSmem) continue;
+        best = around * rows * slabs;
+        out = BrickGeom{static_cast<uint32_t>(width), static_cast<uint32_t>(by), static_cast<uint32_t>(bz), static_cast<uint32_t>(rows)};
+        blocks = static_cast<uint32_t>(rows * slabs);
+    }
+    return best != 0;
+}
+
+template <bool kSmooth, int kPer>
+bool launch_cg_resident(CgArgs& a, uint32_t resident, cudaStream_t stream, XsStatus& status) {
+    uint32_t blocks = 0;
+    if (!brick_for(a.g, resident, kPer, kSmooth, a.brick, blocks)) return false;
+    status = launch_cg<kSmooth, kPer>(a, blocks, brick_smem(a.brick.row_quads, a.brick.by, a.brick.bz, kPer, kSmooth), stream);
+    return true;
+}
+
+// Which form serves a grid (B200, us per iteration, plain solve; the two-pass
+// kernel before -> now):
+//  * resident, up to 148 x 512 x 4 groups (1.2 M cells): 32x48x32 10.7 -> 4.0,
+//    64^3 13.5 -> 4.0, 100x75x90 20 -> 7.8 (with a mask 36 -> 7.9), 96^3 21 ->
+//    7.5;
+//  * marching above, where the two-pass kernel has no 4-cell path (colliders,
+//    rows that are no multiple of 4): 130^3 57 -> 21, masked 200x190x180 280 ->
+//    175; and for plain solves up to 2.5 M cells where it has one: 112^3 22.9 ->
+//    16.2, 128^3 26 -> 21.  From 144^3 on, and for warm starts of a dozen
+//    iterations (128^3: 0.42 against 0.48 ms), the two-pass kernel's lighter
+//    set-up and larger occupancy win: 160^3 36 against 38, 256^3 120 against 141;
+//  * false: neither (rows of more than 764 cells leave the marching form's
+//    runs too short, thin grids the padding too large).
+template <bool kSmooth>
+bool launch_cg_any(CgArgs& a, int sms, cudaStream_t stream, XsStatus& status) {
+    const uint32_t resident = std::min<uint32_t>(kMaxCgBlocks, static_cast<uint32_t>(sms));
+    if (launch_cg_resident<kSmooth, 1>(a, resident, stream, status) || launch_cg_resident<kSmooth, 2>(a, resident, stream, status) ||
+        launch_cg_resident<kSmooth, 3>(a, resident, stream, status) || launch_cg_resident<kSmooth, 4>(a, resident, stream, status))
+        return true;
+    if (a.c.use_fast && (kSmooth || a.g.n > 2500000u)) return false;
+    constexpr uint32_t span = kMarchPer * kCgThreads;
+    const uint32_t halo = a.g.pitch / 4, plane_quads = halo * a.g.ny;
+    if (8 * halo > 3 * span) return false;
+    const uint32_t most = span - 2 * halo;
+    // equal runs; the slabs that leave the least work to the busiest block (a
+    // slab's ends cost about a plane and a half)
+    a.runs = (plane_quads + most - 1) / most;
+    a.run = (plane_quads + a.runs - 1) / a.runs;
+    float best = 0.0f;
+    for (uint32_t slab = a.g.nz; slab >= 1; --slab) {
+        const uint32_t slabs = (a.g.nz + slab - 1) / slab, rounds = (a.runs * slabs + resident - 1) / resident;
+        const float cost = static_cast<float>(rounds) * (static_cast<float>(slab) + 1.5f);
+        if (best == 0.0f || cost < best) {
+            best = cost;
+            a.slab = slab;
+            a.slabs = slabs;
+        }
+    }
+    status = launch_cg<kSmooth, 0>(a, std::min(resident, a.runs * a.slabs), 3ull * span * sizeof(float4), stream);
+    return true;
+}
+
 }  // namespace
 
 XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolve& solve, uint32_t anchor, const uint32_t* mask,
@@ -1238,6 +1379,24 @@ XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolv
     a.use_fast = (mask == nullptr && g.nx % 4 == 0 && n < (1ull << 31)) ? 1u : 0u;
     if (a.use_fast) a.fast = fast_geom(g, anchor, pb);
     a.fast_residual = (a.use_fast && fast_pass_ok(g, mask, anchor, pb, rhs_d == nullptr)) ? 1u : 0u;
+    if (w.padded) {
+        CgArgs b{};
+        b.c = a;
+        b.g = pad_geom(g, pb);
+        b.z[0] = w.z;
+        b.z[1] = w.z1;
+        b.p[0] = w.p0;
+        b.p[1] = w.p1;
+        b.q[0] = w.q;
+        b.q[1] = w.q1;
+        b.e = w.e;
+        b.s = w.s;
+        b.y = w.y;
+        b.code = w.code;
+        b.slots = static_cast<ulonglong2*>(w.slots);
+        XsStatus done = XS_OK;
+        if (a.smooth ? launch_cg_any<true>(b, lim.sms, stream, done) : launch_cg_any<false>(b, lim.sms, stream, done)) return done;
+    }
     const unsigned fast_blocks = persistent_blocks(lim.pcg_fast_blocks_per_sm[a.smooth], lim.sms, n / 4);
     const unsigned blocks = persistent_blocks(lim.pcg_blocks_per_sm[a.smooth], lim.sms, n);
     if (a.use_fast)

@@ -21,6 +21,7 @@ struct SolverState {
 struct PressureWorkspace {
     SolverState* state;
     double* partials;
+    void* slots;  // sums of the single-synchronisation PCG, zeroed before each solve
     double* x64;  // FP64 solution iterate (also the reverse-sweep hand-off)
     float* z;     // preconditioned residual r / diag
     float* p0;
@@ -29,8 +30,22 @@ struct PressureWorkspace {
     float* e;     // FP32 correction of the current CG pass
     float* s;     // minimal-residual smoothed residual (warm starts)
     float* y;     // smoothed correction (warm starts)
+    float* z1;    // second copies of z and q, and the cell codes: the padded
+    float* q1;    // vectors of the single-synchronisation PCG (null on grids
+    uint8_t* code;  // it does not serve)
+    bool padded;
     size_t bytes;
 };
+
+// Floats per vector when rows and planes are padded (pcg_single.cuh), and
+// whether that is worth its memory: thin grids, which would multiply it,
+// keep the unpadded solver.
+uint64_t padded_cells(const Grid& g, const uint32_t (&modes)[6]);
+constexpr uint64_t padded_limit(uint64_t cells) { return cells + cells / 4 + 16384; }
+// One block of slots per resident CTA (one on each SM), two sets, up to 16
+// sums of 16 bytes each.
+constexpr int kMaxCgBlocks = 160;
+constexpr size_t kSlotBytes = 2ull * kMaxCgBlocks * 16 * 16;
 
 // Division by a runtime constant for numerators below 2^31:
 // q = (n * m) >> shift with m = floor(2^shift / d) + 1, shift = 31 + ceil(log2 d).

@@ -7,14 +7,14 @@
 // allocation could fail or stall at an inconvenient time.  The regular
 // xs_pressure_solve needs a caller-provided workspace; this variant instead
 // keeps its scratch (solver control block, reduction slots, the FP64
-// iterate and the seven FP32 vectors of the CG and smoothing recurrences) in
-// one statically sized array in device memory that belongs to the library.
+// iterate and the nine padded FP32 vectors of the CG and smoothing
+// recurrences) in one statically sized array in device memory that belongs to the library.
 //
 // Limits and sharing:
 //  * At most XS_STATIC_SOLVE_MAX_CELLS cells; larger grids are rejected with
 //    XS_CAPACITY_EXCEEDED before anything is launched.
 //  * The array is part of this file's device module: each GPU on which the
-//    entry point is used holds it (about 9.1 MiB at the 64^3 limit) until the
+//    entry point is used holds it (about 15 MiB at the 64^3 limit) until the
 //    process exits.
 //  * All calls on a device share the one array and it keeps whatever the
 //    last call left in it; the solver zeroes its control block at the start
@@ -43,7 +43,8 @@ constexpr size_t round256(size_t v) { return (v + 255) / 256 * 256; }
 constexpr uint64_t kStaticMaxCells = XS_STATIC_SOLVE_MAX_CELLS;
 // Same carving as carve_pressure_workspace for the largest admitted grid.
 constexpr size_t kStaticBytes = round256(sizeof(SolverState)) + round256(sizeof(double) * kPartialSlots * kMaxPersistentBlocks) +
-                                round256(sizeof(double) * kStaticMaxCells) + 7 * round256(sizeof(float) * kStaticMaxCells);
+                                round256(kSlotBytes) + round256(sizeof(double) * kStaticMaxCells) +
+                                9 * round256(sizeof(float) * padded_limit(kStaticMaxCells)) + round256(padded_limit(kStaticMaxCells));
 
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticBytes];
 

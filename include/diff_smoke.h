@@ -232,9 +232,9 @@ XsStatus xs_pressure_solve(cudaStream_t stream, XsGrid grid, const XsPressureSol
  * that only hand over their input and output buffers, or that forbid
  * allocations outside their own pool): it takes no workspace and calls no
  * allocator; its scratch is one library-owned device array sized for at
- * most XS_STATIC_SOLVE_MAX_CELLS cells (about 9.1 MiB: seven FP32 vectors
- * plus the FP64 iterate at 64^3, held by each GPU the entry point runs on
- * until the process exits).  Larger grids return XS_CAPACITY_EXCEEDED
+ * most XS_STATIC_SOLVE_MAX_CELLS cells (about 15 MiB: nine padded FP32
+ * vectors, a byte per cell and the FP64 iterate at 64^3, held by each GPU the
+ * entry point runs on until the process exits).  Larger grids return XS_CAPACITY_EXCEEDED
  * without launching.  All calls share that array: calls that overlap on the
  * GPU race, so order them on one stream.  The first call on a device
  * resolves the array's address (make it before any stream capture).
