@@ -600,7 +600,12 @@ XsStatus projection_vjp(cudaStream_t st, const Grid& g, const XsPressureSolve& s
         adj.scale_guess = 0u;
         const bool ring = history && history->history > 0;
         const bool coarse = ring && history->coarsening != 0 && mask == nullptr;
-        if (ring) {
+        DirectPlan plan;
+        float* low = nullptr;
+        const bool direct = coarse && history->direct && direct_plan(g, mask, anchor, pb, false, plan);
+        if (direct) {  // the grid's operator separates: solved as it is
+            if ((s = direct_start<double>(st, g, pb, *history, plan, pa, &adj.initial_guess, &low)) != XS_OK) return s;
+        } else if (ring) {
             // successive adjoint solves of a reverse pass are related: Galerkin
             // start from the ring of previous adjoint solutions, then (with
             // coarsening) kAdjointStartCycles rounds of sweeps and an
@@ -615,9 +620,9 @@ XsStatus projection_vjp(cudaStream_t st, const Grid& g, const XsPressureSolve& s
                 adj.initial_guess = x;
             }
         }
-        s = solve_pressure(st, g, adj, anchor, mask, pb, nullptr, pa, nullptr, ra, workspace, nullptr);
-        if (s == XS_OK && coarse) s = record_coarse_iterations(st, *history, workspace, g);
-        if (s == XS_OK && ring) s = history_push(st, g, anchor, mask, pb, *history, nullptr, ra);
+        s = solve_pressure(st, g, adj, anchor, mask, pb, nullptr, pa, nullptr, ra, workspace, nullptr, low);
+        if (s == XS_OK && coarse && !direct) s = record_coarse_iterations(st, *history, workspace, g);
+        if (s == XS_OK && ring && !direct) s = history_push(st, g, anchor, mask, pb, *history, nullptr, ra);
     }
     if (s != XS_OK) return s;
     const uint64_t f0 = face_count(g, 0), f1 = face_count(g, 1), f2 = face_count(g, 2);

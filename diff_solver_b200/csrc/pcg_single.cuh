@@ -277,7 +277,7 @@ __device__ __noinline__ void residual_to(const PcgArgs& c, const Store& out, int
             float4 d4;
             const uint32_t row = fastdiv(i, f.dnx), z = fastdiv(row, f.dny), y = row - z * f.ny, x = i - row * f.nx;
             if (mode == kFromGuess) {
-                apply4_fp64(f, c.guess, i, xi, ax, d4);
+                apply4_fp64(f, guess_view(c), i, xi, ax, d4);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
                     xi[k] *= scale;
@@ -319,11 +319,12 @@ __device__ __noinline__ void residual_to(const PcgArgs& c, const Store& out, int
         const double b = act ? rhs_at(c, i) + static_cast<double>(s.fixed_sum) : 0.0;
         double xi = 0.0, ax = 0.0;
         if (act && mode == kFromGuess) {
-            xi = c.guess[i];
+            const GuessView guess = guess_view(c);
+            xi = guess[i];
             ax = s.diag * xi;
 #pragma unroll
             for (int f = 0; f < 6; ++f)
-                if ((s.conn >> f) & 1u) { const uint64_t j = s.nb[f]; if (j != c.op.anchor) ax -= static_cast<double>(c.guess[j]); }
+                if ((s.conn >> f) & 1u) { const uint64_t j = s.nb[f]; if (j != c.op.anchor) ax -= guess[j]; }
             xi *= scale;
             ax *= scale;
         } else if (act && mode == kFromX64) {

@@ -231,6 +231,7 @@ struct PcgArgs {
     const float* rhs_f;   // forward right-hand side (FP32), or
     const double* rhs_d;  // adjoint right-hand side (FP64)
     const float* guess;   // warm start or null
+    const float* guess_low;  // added to it in FP64 (null: none)
     uint32_t scale_guess; // start from alpha * guess, alpha = (g.b) / (g.A g)
     double* x64;
     float* z;
@@ -253,6 +254,16 @@ struct PcgArgs {
 
 enum ResidualMode { kFromZero = 0, kFromGuess = 1, kFromX64 = 2 };
 
+// The guess as the FP64 sum of its two parts.
+struct GuessView {
+    const float *high, *low;
+    __device__ __forceinline__ double operator[](uint64_t i) const {
+        const double v = high[i];
+        return low ? v + static_cast<double>(low[i]) : v;
+    }
+};
+__device__ __forceinline__ GuessView guess_view(const PcgArgs& a) { return GuessView{a.guess, a.guess_low}; }
+
 __device__ __forceinline__ double rhs_at(const PcgArgs& a, uint64_t i) {
     return a.rhs_d ? a.rhs_d[i] : static_cast<double>(a.rhs_f[i]);
 }
@@ -269,11 +280,12 @@ __device__ void guess_energy_phase(const PcgArgs& a, double (&v)[2]) {
         decode(i, g.nx, g.ny, x, y, z);
         CellStencil s;
         if (!stencil(a.op, x, y, z, i, s)) continue;
-        const double gi = a.guess[i];
+        const GuessView guess = guess_view(a);
+        const double gi = guess[i];
         double ag = s.diag * gi;
 #pragma unroll
         for (int f = 0; f < 6; ++f)
-            if ((s.conn >> f) & 1u) { const uint64_t j = s.nb[f]; if (j != a.op.anchor) ag -= static_cast<double>(a.guess[j]); }
+            if ((s.conn >> f) & 1u) { const uint64_t j = s.nb[f]; if (j != a.op.anchor) ag -= guess[j]; }
         v[0] += gi * (rhs_at(a, i) + static_cast<double>(s.fixed_sum));
         v[1] += gi * ag;
     }
@@ -301,11 +313,12 @@ __device__ void residual_phase(const PcgArgs& a, int mode, double (&v)[3], doubl
         const double b = rhs_at(a, i) + static_cast<double>(s.fixed_sum);
         double xi = 0.0, ax = 0.0;
         if (mode == kFromGuess) {
-            xi = a.guess[i];
+            const GuessView guess = guess_view(a);
+            xi = guess[i];
             ax = s.diag * xi;
 #pragma unroll
             for (int f = 0; f < 6; ++f)
-                if ((s.conn >> f) & 1u) { const uint64_t j = s.nb[f]; if (j != a.op.anchor) ax -= static_cast<double>(a.guess[j]); }
+                if ((s.conn >> f) & 1u) { const uint64_t j = s.nb[f]; if (j != a.op.anchor) ax -= guess[j]; }
             xi *= scale;
             ax *= scale;
             a.x64[i] = xi;
@@ -749,6 +762,18 @@ __global__ void fast_pass_kernel(FastGeom f, const float* __restrict__ x, const 
     }
 }
 
+// out = b - A x with the products in FP64: the residual of an almost exact x,
+// which the rounding of an FP32 A x would drown.
+template <class T>
+__global__ void fast_residual64_kernel(FastGeom f, const float* __restrict__ x, const T* __restrict__ rhs, float* __restrict__ out) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < f.groups; t += gridDim.x * blockDim.x) {
+        const uint32_t i = 4u * t;
+        float4 c, d;
+        const Double4 q = apply4(f, x, i, c, d), b = ld4_rhs(rhs + i);
+        st4(out + i, round4(Double4{b.x - q.x, b.y - q.y, b.z - q.z, b.w - q.w}));
+    }
+}
+
 // residual_phase on the fast path for grids without an anchor cell and with
 // no non-zero fixed boundary values (then every cell is an unknown and b is
 // the right-hand side alone): 4 cells of a row per thread, the same FP64
@@ -757,15 +782,15 @@ __device__ __forceinline__ double rhs_at4(const PcgArgs& a, uint32_t i, int k) {
     return a.rhs_d ? a.rhs_d[i + k] : static_cast<double>(a.rhs_f[i + k]);
 }
 
-template <class T>
-__device__ __forceinline__ void load_x4(const T* __restrict__ v, uint32_t i, double (&c)[4]) {
+template <class View>
+__device__ __forceinline__ void load_x4(const View& v, uint32_t i, double (&c)[4]) {
 #pragma unroll
     for (int k = 0; k < 4; ++k) c[k] = static_cast<double>(v[i + k]);
 }
 
-// A x for the 4 cells at i: x is the guess (FP32) or the FP64 iterate.
-template <class T>
-__device__ __forceinline__ void apply4_fp64(const FastGeom& f, const T* __restrict__ x, uint32_t i, double (&c)[4], double (&ax)[4],
+// A x for the 4 cells at i: x is the guess or the FP64 iterate.
+template <class View>
+__device__ __forceinline__ void apply4_fp64(const FastGeom& f, const View& x, uint32_t i, double (&c)[4], double (&ax)[4],
                                             float4& d) {
     const uint32_t row = fastdiv(i, f.dnx);
     const uint32_t x0 = i - row * f.nx;
@@ -802,7 +827,7 @@ __device__ void residual_fast(const PcgArgs& a, const FastGeom& f, int mode, dou
         double xi[4] = {0.0, 0.0, 0.0, 0.0}, ax[4] = {0.0, 0.0, 0.0, 0.0};
         float4 d4;
         if (mode == kFromGuess) {
-            apply4_fp64(f, a.guess, i, xi, ax, d4);
+            apply4_fp64(f, guess_view(a), i, xi, ax, d4);
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 xi[k] *= scale;
@@ -1336,7 +1361,7 @@ bool launch_cg_any(CgArgs& a, int sms, cudaStream_t stream, XsStatus& status) {
 
 XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolve& solve, uint32_t anchor, const uint32_t* mask,
                         const XsScalarBoundary& pb, const float* rhs_f, const double* rhs_d, float* pressure_out,
-                        double* solution_out, void* workspace, PressureWorkspace* carved) {
+                        double* solution_out, void* workspace, PressureWorkspace* carved, const float* guess_low) {
     if (!workspace) return XS_INVALID_ARGUMENT;
     const PressureWorkspace w = carve_pressure_workspace(workspace, g);
     if (carved) *carved = w;
@@ -1357,6 +1382,7 @@ XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolv
     a.rhs_f = rhs_f;
     a.rhs_d = rhs_d;
     a.guess = solve.initial_guess;
+    a.guess_low = solve.initial_guess ? guess_low : nullptr;
     a.scale_guess = solve.scale_guess;
     // residual smoothing pays off from warm starts (2-4x fewer iterations at
     // 128^3); from zero it saves ~4 % of the iterations for 44 % more traffic
@@ -1795,6 +1821,7 @@ uint32_t second_coarsening(const Grid& coarse) {
     return 0;
 }
 
+static bool direct_fits(const Grid& g) { return g.nx <= kDirectMax && g.ny <= kDirectMax && g.nz <= kDirectMax; }
 static bool spectral_fits(const Grid& c) { return c.nx <= kSpectralMax && c.ny <= kSpectralMax && c.nz <= kSpectralMax; }
 
 size_t warm_history_bytes(const Grid& g, uint32_t history, uint32_t coarsening) {
@@ -1806,6 +1833,7 @@ size_t warm_history_bytes(const Grid& g, uint32_t history, uint32_t coarsening) 
     if (coarse_grid(g, coarsening, c)) {
         const size_t nc = cell_count(c);
         bytes += align_up(n * 4, 256) + align_up(nc * 8, 256) + align_up(nc * 4, 256) + align_up(pressure_workspace_bytes(c), 256);
+        if (direct_fits(g)) bytes += align_up(direct_basis_bytes(), 256);
         if (spectral_fits(c)) bytes += align_up(4 * 6 * kSpectralMax * kSpectralMax, 256) + align_up(4 * 3 * kSpectralMax, 256);
         const uint32_t f2 = second_coarsening(c);
         if (f2 && coarse_grid(c, f2, c2)) {
@@ -1846,6 +1874,7 @@ WarmHistory carve_warm_history(void* base, const Grid& g, uint32_t history, uint
         h.coarse_rhs = reinterpret_cast<double*>(take(nc * 8));
         h.coarse_solution = reinterpret_cast<float*>(take(nc * 4));
         h.coarse_solver = take(pressure_workspace_bytes(h.coarse));
+        if (direct_fits(g)) h.direct = take(direct_basis_bytes());
         if (spectral_fits(h.coarse)) {
             h.spectral_basis = reinterpret_cast<float*>(take(4 * 6 * kSpectralMax * kSpectralMax));
             h.spectral_eigen = reinterpret_cast<float*>(take(4 * 3 * kSpectralMax));
@@ -2295,6 +2324,39 @@ XsStatus start_residual(cudaStream_t st, const Grid& g, uint32_t anchor, const u
     }
     return check_launch();
 }
+
+// Above the grids the solve keeps resident an iteration costs more than a
+// tenth of a direct solve: a second one on the rounding residual of the first
+// (in FP64, added in FP64) leaves nothing to do.  Initial residual and fine
+// iterations with one -> two: 128^3 2.7e-4, 14 -> 4e-10, 0; 256^3 9e-4, 53 ->
+// 2e-9, 0.  Below, one leaves 6 to 8 iterations of 4 to 8 us (96x80x64,
+// 146x100x56), about what the second would take.
+constexpr uint64_t kDirectTwice = 1200000;
+
+template <class T>
+XsStatus direct_start(cudaStream_t st, const Grid& g, const XsScalarBoundary& pb, const WarmHistory& h, const DirectPlan& plan, const T* rhs,
+                      const float** guess, float** low) {
+    XsStatus s = direct_solve<T>(st, g, plan, rhs, h.extra_product, h.correction, h.ring_start, h.direct);
+    *guess = h.ring_start;
+    *low = nullptr;
+    const uint64_t n = cell_count(g);
+    if (s != XS_OK || n < kDirectTwice) return s;
+    const uint32_t none = static_cast<uint32_t>(n);  // no anchor cell
+    if (fast_pass_ok(g, nullptr, none, pb, false)) {
+        fast_residual64_kernel<T><<<fast_pass_blocks(g), 256, 0, st>>>(fast_geom(g, none, pb), h.ring_start, rhs, h.residual);
+    } else {
+        const Operator op{g, nullptr, none, pb, false};
+        start_residual_kernel<T><<<static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 148 * 16)), 256, 0, st>>>(op, rhs, h.ring_start, h.residual);
+    }
+    if ((s = check_launch()) != XS_OK) return s;
+    *low = h.start;
+    return direct_solve<float>(st, g, plan, h.residual, h.extra_product, h.correction, h.start, h.direct);
+}
+
+template XsStatus direct_start<float>(cudaStream_t, const Grid&, const XsScalarBoundary&, const WarmHistory&, const DirectPlan&, const float*,
+                                      const float**, float**);
+template XsStatus direct_start<double>(cudaStream_t, const Grid&, const XsScalarBoundary&, const WarmHistory&, const DirectPlan&, const double*,
+                                       const float**, float**);
 
 XsStatus history_push(cudaStream_t st, const Grid& g, uint32_t anchor, const uint32_t* mask, const XsScalarBoundary& pb, const WarmHistory& h,
                       const float* pressure, const double* pressure64) {

@@ -70,10 +70,11 @@ size_t pressure_workspace_bytes(const Grid& g);
 // Solves the pressure system for rhs_f (forward, FP32, fixed boundary values
 // enter b) or rhs_d (adjoint, FP64, no fixed values).  pressure_out receives
 // an FP32 copy, solution_out an FP64 copy (either may be null); the FP64
-// iterate stays in the workspace (carved->x64).
+// iterate stays in the workspace (carved->x64).  guess_low: added to the
+// initial guess in FP64.
 XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolve& solve, uint32_t anchor, const uint32_t* mask,
                         const XsScalarBoundary& pb, const float* rhs_f, const double* rhs_d, float* pressure_out,
-                        double* solution_out, void* workspace, PressureWorkspace* carved);
+                        double* solution_out, void* workspace, PressureWorkspace* carved, const float* guess_low = nullptr);
 
 // The reference's reversed red-black sweeps (operators.cu:1025-1028).
 XsStatus reverse_rbgs(cudaStream_t stream, const Grid& g, uint32_t sweeps, uint32_t anchor, const uint32_t* mask,
@@ -121,7 +122,23 @@ struct WarmHistory {
     // eigenbases of the coarse grid's axes (coarse grids within kSpectralMax)
     float* spectral_basis;    // 6 kSpectralMax^2 (each axis' basis and its transpose)
     float* spectral_eigen;    // 3 kSpectralMax
+    void* direct;             // bases of the fine grid's direct solve (grids within kDirectMax)
 };
+// Direct solve on the fluid grid itself (direct.cu): up to kDirectMax cells
+// per axis, no colliders, no anchor cell, no fixed boundary values in b
+// (fixed_values: b has them where they are not 0); two axes, x among them,
+// with equal ends or periodic, the third not periodic.
+constexpr int kDirectMax = 512;
+struct DirectPlan {
+    int axis, other;           // the tridiagonal axis, and the transformed one besides x
+    int kind_x, kind_other;
+    int fixed_lo, fixed_hi;    // ends of the tridiagonal axis
+};
+bool direct_plan(const Grid& g, const uint32_t* mask, uint32_t anchor, const XsScalarBoundary& pb, bool fixed_values, DirectPlan& plan);
+size_t direct_basis_bytes();
+// x = A^-1 rhs in FP32; tmp, tmp2: scratch (N), x may be tmp2.
+template <class T>
+XsStatus direct_solve(cudaStream_t st, const Grid& g, const DirectPlan& plan, const T* rhs, float* tmp, float* tmp2, float* x, void* basis);
 // Exact coarse solve for operators that separate by axis (spectral.cu):
 // grids of at most kSpectralMax cells per axis, no anchor cell, no colliders.
 constexpr int kSpectralMax = 256;
@@ -135,6 +152,13 @@ bool spectral_axes(const Grid& c, const XsScalarBoundary& pb, uint32_t anchor, S
 // x = A^-1 rhs on grid c by the axes' eigenbases (built into basis /
 // eigen: 6 kSpectralMax^2 and 3 kSpectralMax floats).
 XsStatus spectral_solve(cudaStream_t st, const Grid& c, const SpectralAxes& ax, float* basis, float* eigen, const double* rhs, float* x);
+// The start of a warm-started solve by it: the solution of A x = rhs in two
+// parts, *guess and, on grids past kDirectTwice cells, *low (else null), in
+// h.ring_start and h.start.  h.residual: the residual of the first part
+// alone, where there is a second.
+template <class T>
+XsStatus direct_start(cudaStream_t st, const Grid& g, const XsScalarBoundary& pb, const WarmHistory& h, const DirectPlan& plan, const T* rhs,
+                      const float** guess, float** low);
 constexpr double kCoarseTolerance = 1e-2;
 constexpr uint32_t kCoarseMaxIterations = 1000;
 // Damped Jacobi sweeps (weight 2/3) on the start before its residual is

@@ -39,9 +39,31 @@ XsStatus projection_forward(cudaStream_t st, const Grid& g, const XsPressureSolv
     //    CG removes in a few iterations), and measured 1.3-2x more CG
     //    iterations at 256^3;
     //  * network alone: its guess for b, scaled by the energy-optimal factor.
-    float* guess = nullptr;
+    float *guess = nullptr, *low = nullptr;
     const bool coarse = ring && history->coarsening != 0 && mask == nullptr;
-    if (ring) {
+    DirectPlan plan;
+    const bool direct = coarse && history->direct && history->forward_rounds == 0 && direct_plan(g, mask, anchor, pb, true, plan);
+    if (direct) {
+        // the grid's operator separates: solved as it is, instead of the ring
+        // and the rounds (unless the caller set their number); the network's
+        // step then works on the residual this leaves
+        const WarmHistory& h = *history;
+        const float* x = nullptr;
+        if ((s = direct_start<float>(st, g, pb, h, plan, rhs, &x, &low)) != XS_OK) return s;
+        if (warm_start) {
+            // the residual of both parts is the first part's less A low
+            const float *b = low ? h.residual : rhs, *y = low ? low : x;
+            XsScalarBoundary plain = pb;
+            for (float& v : plain.values) v = 0.0f;
+            if ((s = start_residual(st, g, anchor, mask, plain, b, y, h.correction)) != XS_OK) return s;
+            if ((s = warm_start_guess(warm_start, st, g, h.correction, &guess)) != XS_OK) return s;
+            float* to = low ? low : h.start;
+            if ((s = line_step(st, g, anchor, mask, pb, h, guess, y, h.correction, to, false)) != XS_OK) return s;
+            if (!low) x = to;
+        }
+        used.initial_guess = x;
+        used.scale_guess = 0u;
+    } else if (ring) {
         const WarmHistory& h = *history;
         if ((s = galerkin_combine(st, g, anchor, mask, pb, h, true, nullptr, 0, rhs, h.ring_start)) != XS_OK) return s;
         used.initial_guess = h.ring_start;
@@ -71,11 +93,11 @@ XsStatus projection_forward(cudaStream_t st, const Grid& g, const XsPressureSolv
         used.scale_guess = 1u;
     }
     if ((s = mark_stage(st, stages, 1)) != XS_OK) return s;
-    s = solve_pressure(st, g, used, anchor, mask, pb, rhs, nullptr, pressure, nullptr, workspace, &w);
+    s = solve_pressure(st, g, used, anchor, mask, pb, rhs, nullptr, pressure, nullptr, workspace, &w, low);
     if (s != XS_OK) return s;
     if ((s = mark_stage(st, stages, 2)) != XS_OK) return s;
-    if (coarse && (s = record_coarse_iterations(st, *history, workspace, g)) != XS_OK) return s;
-    if (ring && (s = history_push(st, g, anchor, mask, pb, *history, pressure)) != XS_OK) return s;
+    if (coarse && !direct && (s = record_coarse_iterations(st, *history, workspace, g)) != XS_OK) return s;
+    if (ring && !direct && (s = history_push(st, g, anchor, mask, pb, *history, pressure)) != XS_OK) return s;
     if (end && cudaEventRecord(end, st) != cudaSuccess) return XS_CUDA_ERROR;
     if ((s = mark_stage(st, stages, 3)) != XS_OK) return s;
     s = solve.kind == XS_SOLVER_RED_BLACK_GAUSS_SEIDEL ? launch_project(st, g, mask, u, pressure, out) : launch_project64(st, g, mask, u, w.x64, out);

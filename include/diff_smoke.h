@@ -339,11 +339,18 @@ typedef struct XsSmokeModel {
      * solution is interpolated back and the start takes one energy-optimal
      * step along it (before the learned correction's step), in rounds
      * (warm_start_rounds).  It removes the smooth error that fine-grid CG
-     * reduces slowest. */
+     * reduces slowest.
+     * Where the fluid grid's own operator separates (no anchor cell, no fixed
+     * boundary value other than 0, at most 512 cells per axis, equal ends or
+     * periodic x and y or z, the third axis not periodic) and
+     * warm_start_rounds is 0, the system is solved there directly instead, in
+     * FP32, and neither ring nor rounds are used; the learned correction then
+     * works on the residual that leaves. */
     uint32_t warm_start_coarsening;
     /* rounds of sweeps and coarse-grid correction before a forward solve
      * (0: the defaults, two without a learned warm start and one before its
-     * step; at most 8).  Adjoint solves always take three. */
+     * step, or the direct solve above; at most 8).  Adjoint solves take the
+     * direct solve or three. */
     uint32_t warm_start_rounds;
     /* optional per-stage timing of xs_smoke_forward_step (NULL: none): an
      * array of XS_STEP_STAGES + 1 events created by the caller with timing
