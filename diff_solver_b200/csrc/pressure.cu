@@ -1051,15 +1051,8 @@ struct RbgsArgs {
     SolverState* st;
 };
 
-__global__ void __launch_bounds__(kBlock) rbgs_kernel(RbgsArgs a) {
-    __shared__ double red[4 * 32];
-    for (uint32_t it = 0; it < a.sweeps; ++it) {
-        rbgs_phase(a.op, 0, a.rhs, a.p);
-        if (!grid_barrier(a.st, a.partials, red)) return;
-        rbgs_phase(a.op, 1, a.rhs, a.p);
-        if (!grid_barrier(a.st, a.partials, red)) return;
-    }
-    // report the relative residual reached, in FP64
+// The relative residual reached, in FP64.
+__device__ __forceinline__ void rbgs_report(const RbgsArgs& a, double* red) {
     const Grid& g = a.op.g;
     const uint64_t n = cell_count(g);
     double v[2] = {0.0, 0.0};
@@ -1089,6 +1082,23 @@ __global__ void __launch_bounds__(kBlock) rbgs_kernel(RbgsArgs a) {
         a.st->stats.final_residual = v[0] > 0.0 ? sqrt(v[1] / v[0]) : 0.0;
     }
 }
+
+__global__ void __launch_bounds__(kBlock) rbgs_kernel(RbgsArgs a) {
+    __shared__ double red[4 * 32];
+    for (uint32_t it = 0; it < a.sweeps; ++it) {
+        rbgs_phase(a.op, 0, a.rhs, a.p);
+        if (!grid_barrier(a.st, a.partials, red)) return;
+        rbgs_phase(a.op, 1, a.rhs, a.p);
+        if (!grid_barrier(a.st, a.partials, red)) return;
+    }
+    rbgs_report(a, red);
+}
+
+}  // namespace xs
+
+#include "rbgs_resident.cuh"
+
+namespace xs {
 
 // Reverse sweeps (operators.cu:935-955) in gather form: the cells of one
 // parity hand lambda_p / diag to the right-hand-side adjoint and to their
@@ -1359,6 +1369,70 @@ bool launch_cg_any(CgArgs& a, int sms, cudaStream_t stream, XsStatus& status) {
 
 }  // namespace
 
+namespace {
+
+// The brick of whole rows, one per SM, that leaves each thread at most kPer
+// groups per colour and the least surface.
+bool rbgs_brick(const Grid& g, uint32_t resident, int per, RbgsBrick& out) {
+    const uint64_t hold = static_cast<uint64_t>(per) * kRbgsThreads, quads = (g.nx + 7ull) / 8ull;
+    uint64_t best = 0;
+    for (uint64_t by = 1; by <= static_cast<uint64_t>(g.ny) && quads * by <= hold; ++by) {
+        uint64_t bz = std::min<uint64_t>(static_cast<uint64_t>(g.nz), hold / (quads * by));
+        const uint64_t slabs = (g.nz + bz - 1) / bz;
+        bz = (g.nz + slabs - 1) / slabs;
+        const uint64_t rows = (g.ny + by - 1) / by;
+        const RbgsBrick b{static_cast<uint32_t>(quads), static_cast<uint32_t>(by), static_cast<uint32_t>(bz), static_cast<uint32_t>(rows),
+                          static_cast<uint32_t>(slabs)};
+        if (rows * slabs > resident || rbgs_smem(b) > kCgMaxSmem) continue;
+        const uint64_t cost = quads * by * bz + 2 * quads * (by + bz);  // a block's groups and the ones it is handed
+        if (best != 0 && cost >= best) continue;
+        best = cost;
+        out = b;
+    }
+    return best != 0;
+}
+
+template <int kPer>
+XsStatus launch_rbgs_resident(RbgsResidentArgs& a, cudaStream_t stream) {
+    static DeviceOnce configured;
+    if (!configured.run([] { return cudaFuncSetAttribute(rbgs_resident_kernel<kPer>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kCgMaxSmem)); }))
+        return XS_CUDA_ERROR;
+    const unsigned blocks = a.b.bricks_y * a.b.bricks_z;
+    if (cudaMemsetAsync(a.flags, 0, sizeof(uint32_t) * kRbgsFlagStride * blocks, stream) != cudaSuccess) return XS_CUDA_ERROR;
+    void* params[] = {&a};
+    const cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void*>(rbgs_resident_kernel<kPer>), dim3(blocks), dim3(kRbgsThreads), params,
+                                                      rbgs_smem(a.b), stream);
+    if (e != cudaSuccess) return check_cuda(e);
+    return check_launch();
+}
+
+// Sweeps with the grid in the SMs: up to 148 x 512 x 8 groups of 8 cells (4.8 M
+// cells) whose pressures fit the shared memories; no periodic axis (on an odd
+// one two cells of a colour are neighbours, which the general kernel updates
+// in whatever order they come).  false: the general kernel serves.
+bool launch_rbgs_any(const RbgsArgs& c, const PressureWorkspace& w, int sms, cudaStream_t stream, XsStatus& status) {
+    const Grid& g = c.op.g;
+    if (!w.padded || c.sweeps == 0) return false;
+    for (int d = 0; d < 3; ++d)
+        if (c.op.pb.modes[2 * d] == 2u && c.op.pb.modes[2 * d + 1] == 2u) return false;
+    RbgsResidentArgs a{};
+    a.c = c;
+    a.rim[0] = w.z;
+    a.rim[1] = w.q;
+    a.flags = static_cast<uint32_t*>(w.slots);
+    const uint32_t resident = std::min<uint32_t>(kMaxCgBlocks, static_cast<uint32_t>(sms));
+    if (rbgs_brick(g, resident, 1, a.b)) status = launch_rbgs_resident<1>(a, stream);
+    else if (rbgs_brick(g, resident, 2, a.b)) status = launch_rbgs_resident<2>(a, stream);
+    else if (rbgs_brick(g, resident, 3, a.b)) status = launch_rbgs_resident<3>(a, stream);
+    else if (rbgs_brick(g, resident, 4, a.b)) status = launch_rbgs_resident<4>(a, stream);
+    else if (rbgs_brick(g, resident, 6, a.b)) status = launch_rbgs_resident<6>(a, stream);
+    else if (rbgs_brick(g, resident, 8, a.b)) status = launch_rbgs_resident<8>(a, stream);
+    else return false;
+    return true;
+}
+
+}  // namespace
+
 XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolve& solve, uint32_t anchor, const uint32_t* mask,
                         const XsScalarBoundary& pb, const float* rhs_f, const double* rhs_d, float* pressure_out,
                         double* solution_out, void* workspace, PressureWorkspace* carved, const float* guess_low) {
@@ -1372,8 +1446,9 @@ XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolv
     Operator op{g, mask, anchor, pb, rhs_d == nullptr};
     if (solve.kind == XS_SOLVER_RED_BLACK_GAUSS_SEIDEL) {
         if (!rhs_f || !pressure_out) return XS_INVALID_ARGUMENT;
-        if (cudaMemsetAsync(pressure_out, 0, sizeof(float) * cell_count(g), stream) != cudaSuccess) return XS_CUDA_ERROR;
         RbgsArgs a{op, rhs_f, pressure_out, solve.max_iterations, w.partials, w.state};
+        if (launch_rbgs_any(a, w, lim.sms, stream, s)) return s;
+        if (cudaMemsetAsync(pressure_out, 0, sizeof(float) * cell_count(g), stream) != cudaSuccess) return XS_CUDA_ERROR;
         return launch_cooperative(rbgs_kernel, persistent_blocks(lim.rbgs_blocks_per_sm, lim.sms, cell_count(g)), a, stream);
     }
     if (solve.kind != XS_SOLVER_JACOBI_PCG || !(solve.tolerance >= 0.0)) return XS_INVALID_ARGUMENT;
