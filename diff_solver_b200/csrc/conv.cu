@@ -19,6 +19,7 @@
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cstring>
 #include <mutex>
 
@@ -78,7 +79,6 @@ bool make_weight_map(CUtensorMap* map, const void* base, uint32_t rows, uint32_t
 
 // ------------------------------------------------------------------ forward
 constexpr int kConvThreads = 128;
-constexpr int kStages = 4;
 
 template <int CIN, int COUT>
 struct ConvSmem {
@@ -86,7 +86,9 @@ struct ConvSmem {
     static constexpr uint32_t b_bytes_raw = static_cast<uint32_t>(COUT) * CIN * 2u;
     static constexpr uint32_t b_bytes = (b_bytes_raw + 1023u) / 1024u * 1024u;
     static constexpr uint32_t stage_bytes = a_bytes + b_bytes;
-    static constexpr uint32_t total = 1024u /*alignment slack*/ + kStages * stage_bytes + 256u /*barriers*/;
+    // loads in flight: what 96 KB hold, so that two CTAs fit an SM
+    static constexpr int stages = 98304u / stage_bytes < 12u ? static_cast<int>(98304u / stage_bytes) : 12;
+    static constexpr uint32_t total = 1024u /*alignment slack*/ + stages * stage_bytes + 256u /*barriers*/;
     static constexpr uint32_t tmem_cols = COUT <= 32 ? 32u : 64u;
 };
 
@@ -107,13 +109,13 @@ __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __gri
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
     unsigned char* a_tiles = smem;
-    unsigned char* b_tiles = smem + kStages * L::a_bytes;
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + kStages * L::stage_bytes);
-    uint64_t* empty = full + kStages;
-    uint64_t* accum = empty + kStages;
+    unsigned char* b_tiles = smem + L::stages * L::a_bytes;
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::stages * L::stage_bytes);
+    uint64_t* empty = full + L::stages;
+    uint64_t* accum = empty + L::stages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = static_cast<int>(tc::uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     // tile coordinates
     const uint32_t tiles_x = a.s.x / a.bx, tiles_y = a.s.y / a.by, tiles_z = a.s.z / a.bz;
     uint32_t t = blockIdx.x;
@@ -124,7 +126,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __gri
     const int x0 = static_cast<int>(tx * a.bx), y0 = static_cast<int>(ty * a.by), z0 = static_cast<int>(tz * a.bz);
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < kStages; ++i) {
+        for (int i = 0; i < L::stages; ++i) {
             tc::mbar_init(&full[i], 1);
             tc::mbar_init(&empty[i], 1);
         }
@@ -140,38 +142,40 @@ __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __gri
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = tc::uniform(*tmem_slot);
     bool ok = true;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
         // TMA producer: one stage per tap
-        for (int tap = 0; tap < 27; ++tap) {
-            const int s = tap % kStages, round = tap / kStages;
-            if (tap >= kStages && !tc::mbar_wait(&empty[s], (round - 1) & 1)) { ok = false; break; }
-            tc::mbar_expect_tx(&full[s], L::a_bytes + L::b_bytes_raw);
-            const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
-            tc::tma_load_5d(a_tiles + s * L::a_bytes, &act_map, &full[s], 0, x0 + dx, y0 + dy, z0 + dz, static_cast<int>(b));
-            tc::tma_load_3d(b_tiles + s * L::b_bytes, &w_map, &full[s], 0, 0, tap);
+        if (tc::elect_one()) {
+            for (int tap = 0; tap < 27; ++tap) {
+                const int s = tap % L::stages, round = tap / L::stages;
+                if (tap >= L::stages && !tc::mbar_wait(&empty[s], (round - 1) & 1)) { ok = false; break; }
+                tc::mbar_expect_tx(&full[s], L::a_bytes + L::b_bytes_raw);
+                const int dz = tap / 9 - 1, dy = (tap / 3) % 3 - 1, dx = tap % 3 - 1;
+                tc::tma_load_5d(a_tiles + s * L::a_bytes, &act_map, &full[s], 0, x0 + dx, y0 + dy, z0 + dz, static_cast<int>(b));
+                tc::tma_load_3d(b_tiles + s * L::b_bytes, &w_map, &full[s], 0, 0, tap);
+            }
         }
-    } else if (warp == 1 && lane == 0) {
-        // MMA issuer
+    } else if (warp == 1) {
+        // MMA issuer; the shuffles of uniform() are the whole warp's, before one lane is elected
         constexpr uint32_t idesc = tc::idesc_bf16(128, COUT, false, false);
         constexpr uint32_t row = CIN * 2;
         constexpr uint32_t swz = tc::swizzle_for_row_bytes(row);
-        for (int tap = 0; tap < 27; ++tap) {
-            const int s = tap % kStages, round = tap / kStages;
-            if (!tc::mbar_wait(&full[s], round & 1)) { ok = false; break; }
-            tc::tc_fence_after();
-            const uint32_t a_addr = tc::smem_u32(a_tiles + s * L::a_bytes), b_addr = tc::smem_u32(b_tiles + s * L::b_bytes);
+        const uint64_t a_desc = tc::smem_desc(tc::uniform(tc::smem_u32(a_tiles)), 16u, 8u * row, swz);
+        const uint64_t b_desc = tc::smem_desc(tc::uniform(tc::smem_u32(b_tiles)), 16u, 8u * row, swz);
+        if (tc::elect_one()) {
+            for (int tap = 0; tap < 27; ++tap) {
+                const int s = tap % L::stages, round = tap / L::stages;
+                if (!tc::mbar_wait(&full[s], round & 1)) { ok = false; break; }
+                tc::tc_fence_after();
+                const uint64_t ad = a_desc + (s * L::a_bytes >> 4), bd = b_desc + (s * L::b_bytes >> 4);
 #pragma unroll
-            for (int k = 0; k < CIN / 16; ++k) {
-                const uint64_t ad = tc::smem_desc(a_addr + 32u * k, 16u, 8u * row, swz);
-                const uint64_t bd = tc::smem_desc(b_addr + 32u * k, 16u, 8u * row, swz);
-                tc::mma_bf16(tmem, ad, bd, idesc, (tap > 0 || k > 0) ? 1u : 0u);
+                for (int k = 0; k < CIN / 16; ++k) tc::mma_bf16(tmem, ad + 2u * k, bd + 2u * k, idesc, (tap > 0 || k > 0) ? 1u : 0u);
+                tc::mma_commit(&empty[s]);
             }
-            tc::mma_commit(&empty[s]);
+            tc::mma_commit(accum);
         }
-        tc::mma_commit(accum);
     }
     __syncwarp();
     // epilogue: every warp reads its 32 TMEM lanes (= voxels)
@@ -204,11 +208,264 @@ __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __gri
     if (warp == 0) tc::tmem_dealloc(tmem, L::tmem_cols);
 }
 
+// ------------------------------------------------------------ halo slab
+// The same convolution with the activations read once.  A CTA owns `by` rows
+// of `bz` planes and brings their box, widened by one voxel on every side,
+// into shared memory: planes of voxels in rows of X + 2, a voxel's channels
+// together, 16-byte chunks permuted by their address as the swizzle of that
+// row width does.  That is a K-major operand from any voxel on, so a tap is no
+// more than another start address: (dy (X + 2) + dx) voxels into plane dz.  A
+// tile's 128 rows are consecutive voxels of the widened rows; the two columns
+// between rows are computed too and dropped (at X = 64 and 11 rows 92 % of the
+// products are kept).  The weights are loaded one tap per stage of a ring that
+// holds all 27 of the narrowest layers.
+//
+// What bounds it is the rate at which one warp issues 128 x 16 x 16 MMAs, 40
+// cycles each from uniform registers: 16 -> 16 at 64^3 runs in 26 us (the
+// shifted boxes, 27 x 8.4 MB through L2: 46 to 50), 8 x 64^3 in 159 (294), of
+// which the MMAs are 130.  The unswizzled layout, 8 voxels by 16 bytes at a
+// time, gives the same numbers at a quarter of the operand rate: 140 cycles
+// per MMA.
+//
+constexpr int kSlabThreads = 256;
+
+template <int CIN, int COUT>
+struct SlabSmem {
+    static constexpr uint32_t chunks = CIN / 8;
+    static constexpr uint32_t w_bytes_raw = static_cast<uint32_t>(COUT) * CIN * 2u;
+    static constexpr uint32_t w_bytes = (w_bytes_raw + 1023u) / 1024u * 1024u;
+    // as many taps as 96 KB hold, all 27 but for the widest layers: a stage
+    // filled again costs the MMAs' completion and a load's latency
+    static constexpr int ring = 98304u / w_bytes < 27u ? static_cast<int>(98304u / w_bytes) : 27;
+    static constexpr uint32_t fixed = 1024u /*alignment*/ + ring * w_bytes + 512u /*barriers*/;
+};
+constexpr uint32_t kSlabMaxSmem = 220u * 1024u;
+constexpr uint64_t kSlabMinVoxels = 100000u;
+
+struct SlabPlan {
+    uint32_t by, bz;      // rows and planes of a CTA
+    uint32_t tiles;       // 128-voxel tiles per plane
+    uint32_t voxels;      // voxels of a plane's arrays in shared memory
+    uint32_t columns;     // TMEM columns
+    uint32_t smem;
+};
+
+struct SlabArgs {
+    VolumeShape s;
+    SlabPlan p;
+    const __nv_bfloat16* in;
+    const float* bias;
+    __nv_bfloat16* out;
+    int relu;
+    int* error;
+};
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ SlabArgs a) {
+    using L = SlabSmem<CIN, COUT>;
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* w_ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
+    uint64_t* full = reinterpret_cast<uint64_t*>(w_ring + L::ring * L::w_bytes);
+    uint64_t* empty = full + L::ring;
+    uint64_t* accum = empty + L::ring;
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
+    unsigned char* slab = w_ring + L::ring * L::w_bytes + 512;
+    const int warp = static_cast<int>(tc::uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
+    const uint32_t strips = (a.s.y + a.p.by - 1) / a.p.by, layers = (a.s.z + a.p.bz - 1) / a.p.bz;
+    const uint32_t strip = blockIdx.x % strips, layer = blockIdx.x / strips % layers, b = blockIdx.x / strips / layers;
+    const int y0 = static_cast<int>(strip * a.p.by), z0 = static_cast<int>(layer * a.p.bz);
+    const int rows = min(static_cast<int>(a.p.by), static_cast<int>(a.s.y) - y0), planes = min(static_cast<int>(a.p.bz), static_cast<int>(a.s.z) - z0);
+    const uint32_t px = a.s.x + 2u;
+    constexpr uint32_t row_bytes = CIN * 2u;  // of a voxel
+    const uint32_t plane_bytes = a.p.voxels * row_bytes;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < L::ring; ++i) {
+            tc::mbar_init(&full[i], 1);
+            tc::mbar_init(&empty[i], 1);
+        }
+        tc::mbar_init(accum, 1);
+        tc::fence_barrier_init();
+        tc::prefetch_map(&w_map);
+    }
+    if (warp == 0) {
+        tc::tmem_alloc(tmem_slot, a.p.columns);
+        tc::tmem_relinquish();
+    }
+    __syncthreads();
+    auto load_weights = [&](int tap) {
+        tc::mbar_expect_tx(&full[tap % L::ring], L::w_bytes_raw);
+        tc::tma_load_3d(w_ring + (tap % L::ring) * L::w_bytes, &w_map, &full[tap % L::ring], 0, 0, tap);
+    };
+    if (warp == 0 && tc::elect_one())
+        for (int tap = 0; tap < L::ring; ++tap) load_weights(tap);
+    __syncwarp();
+    // the box, zeros beyond the volume: a warp per row, 16 bytes per lane
+    for (int r = warp; r < (planes + 2) * (rows + 2); r += kSlabThreads / 32) {
+        const int pz = r / (rows + 2), py = r % (rows + 2), z = z0 + pz - 1, y = y0 + py - 1;
+        const bool row_in = y >= 0 && y < static_cast<int>(a.s.y) && z >= 0 && z < static_cast<int>(a.s.z);
+        const __nv_bfloat16* src = a.in + (((static_cast<uint64_t>(b) * a.s.z + (row_in ? z : 0)) * a.s.y + (row_in ? y : 0)) * a.s.x) * CIN;
+        const uint32_t dst = tc::smem_u32(slab) + static_cast<uint32_t>(pz) * plane_bytes + static_cast<uint32_t>(py) * px * row_bytes;
+        for (uint32_t j = lane; j < px * L::chunks; j += 32) {
+            const uint32_t v = j / L::chunks, c = j % L::chunks;
+            const bool in = row_in && v >= 1u && v <= a.s.x;
+            const __nv_bfloat16* from = in ? src + (static_cast<uint64_t>(v) - 1u) * CIN + 8u * c : a.in;
+            const uint32_t at = dst + v * row_bytes + c * 16u;
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(at ^ (((at >> 7) & (L::chunks - 1u)) << 4)), "l"(from),
+                         "r"(in ? 16u : 0u)
+                         : "memory");
+        }
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the box before the tensor pipe's reads of it
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tc::uniform(*tmem_slot);
+    bool ok = true;
+    if (warp == 0) {
+        // the taps past the ring
+        if (L::ring < 27 && tc::elect_one()) {
+            for (int tap = L::ring; tap < 27; ++tap) {
+                if (!tc::mbar_wait(&empty[tap % L::ring], (tap / L::ring - 1) & 1)) { ok = false; break; }
+                load_weights(tap);
+            }
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = tc::idesc_bf16(128, COUT, false, false);
+        constexpr uint32_t w_row = CIN * 2;
+        // descriptors of the box and of the ring; steps in their 16-byte units
+        const uint64_t box = tc::smem_desc(tc::uniform(tc::smem_u32(slab)), 16u, 8u * row_bytes, tc::swizzle_for_row_bytes(row_bytes));
+        const uint64_t weights = tc::smem_desc(tc::uniform(tc::smem_u32(w_ring)), 16u, 8u * w_row, tc::swizzle_for_row_bytes(w_row));
+        constexpr uint32_t tile_step = 128u * row_bytes / 16u;
+        const uint32_t plane_step = plane_bytes / 16u, tiles = a.p.tiles;
+        if (tc::elect_one()) {
+            uint32_t accumulate = 0u;
+            for (int tap = 0; tap < 27; ++tap) {
+                const int s = tap % L::ring, round = tap / L::ring;
+                if (!tc::mbar_wait(&full[s], round & 1)) { ok = false; break; }
+                tc::tc_fence_after();
+                const uint32_t dz = static_cast<uint32_t>(tap) / 9u, dy = static_cast<uint32_t>(tap) / 3u % 3u, dx = static_cast<uint32_t>(tap) % 3u;
+                const uint64_t from = box + dz * plane_step + (dy * px + dx) * (row_bytes / 16u), w = weights + s * (L::w_bytes / 16u);
+#pragma unroll
+                for (uint32_t k = 0; k < CIN / 16; ++k) {
+                    uint32_t d = tmem;
+                    uint64_t plane = from + 2u * k;
+                    for (int z = 0; z < planes; ++z) {
+                        uint64_t tile = plane;
+#pragma unroll 4
+                        for (uint32_t t = 0; t < tiles; ++t) {
+                            tc::mma_bf16(d, tile, w + 2u * k, idesc, accumulate);
+                            tile += tile_step;
+                            d += COUT;
+                        }
+                        plane += plane_step;
+                    }
+                    accumulate = 1u;
+                }
+                tc::mma_commit(&empty[s]);
+            }
+            tc::mma_commit(accum);
+        }
+    }
+    __syncwarp();
+    const bool got = tc::mbar_wait(accum, 0);
+    tc::tc_fence_after();
+    if (got) {
+        // warps 0-3 take the even tiles, 4-7 the odd ones, 32 rows each
+        for (uint32_t i = static_cast<uint32_t>(warp >> 2); i < static_cast<uint32_t>(planes) * a.p.tiles; i += 2u) {
+            const uint32_t pz = i / a.p.tiles, t = i - pz * a.p.tiles;
+            const uint32_t v = t * 128u + static_cast<uint32_t>((warp & 3) * 32 + lane), r = v / px, x = v - r * px;
+            const bool keep = x < a.s.x && r < static_cast<uint32_t>(rows);
+            const uint64_t voxel = ((static_cast<uint64_t>(b) * a.s.z + static_cast<uint32_t>(z0) + pz) * a.s.y + static_cast<uint32_t>(y0) + r) * a.s.x + x;
+            __nv_bfloat16* dst = a.out + voxel * COUT;
+#pragma unroll
+            for (int c0 = 0; c0 < COUT; c0 += 16) {
+                float f[16];
+                tc::tmem_ld16(tmem + (static_cast<uint32_t>((warp & 3) * 32) << 16) + i * COUT + static_cast<uint32_t>(c0), f);
+                __align__(16) __nv_bfloat16 o[16];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) {
+                    float y_ = f[e] + (a.bias ? __ldg(a.bias + c0 + e) : 0.0f);
+                    if (a.relu) y_ = fmaxf(y_, 0.0f);
+                    o[e] = __float2bfloat16(y_);
+                }
+                if (keep) {
+                    reinterpret_cast<uint4*>(dst + c0)[0] = reinterpret_cast<const uint4*>(o)[0];
+                    reinterpret_cast<uint4*>(dst + c0)[1] = reinterpret_cast<const uint4*>(o)[1];
+                }
+            }
+        }
+    }
+    if ((!ok || !got) && a.error) atomicExch(a.error, 1);
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, a.p.columns);
+}
+
+// The rows and planes of a CTA that take the least time on 148 SMs, in cycles:
+// the MMAs (45 each, measured from the issuing warp), the box through L2, the
+// epilogue, and what a wave costs anyway.
+template <int CIN, int COUT>
+bool slab_plan(const VolumeShape& s, SlabPlan& best) {
+    using L = SlabSmem<CIN, COUT>;
+    double least = 0.0;
+    const uint32_t px = s.x + 2u;
+    for (uint32_t bz = 1; bz <= std::min(4u, s.z); ++bz)
+        for (uint32_t by = 1; by <= s.y; ++by) {
+            SlabPlan p{};
+            p.by = by;
+            p.bz = bz;
+            p.tiles = ((by - 1) * px + s.x + 127u) / 128u;
+            p.voxels = std::max((by + 2) * px, p.tiles * 128u + 2u * px + 2u);
+            p.columns = 32u;
+            while (p.columns < bz * p.tiles * COUT) p.columns *= 2;
+            const uint64_t smem = L::fixed + static_cast<uint64_t>(bz + 2) * p.voxels * CIN * 2u;
+            if (p.columns > 512u || smem > kSlabMaxSmem) break;
+            p.smem = static_cast<uint32_t>(smem);
+            const uint64_t ctas = static_cast<uint64_t>(s.batch) * ((s.z + bz - 1) / bz) * ((s.y + by - 1) / by);
+            const double waves = static_cast<double>((ctas + 147) / 148);
+            const double cycles = 27.0 * (bz * p.tiles * (CIN / 16) * 45.0 + 60.0) + smem / 40.0 + bz * p.tiles * 12.0 * COUT + 5000.0;
+            if (least == 0.0 || waves * cycles < least) {
+                least = waves * cycles;
+                best = p;
+            }
+        }
+    return least > 0.0;
+}
+
+template <int CIN, int COUT>
+XsStatus launch_conv_slab(cudaStream_t st, const VolumeShape& s, const SlabPlan& plan, const __nv_bfloat16* in, const __nv_bfloat16* w, const float* bias,
+                          __nv_bfloat16* out, bool relu, int* error) {
+    CUtensorMap wm;
+    // (the box copies are of 16 bytes, as a tensor map's base has to be)
+    if ((reinterpret_cast<uintptr_t>(in) & 15u) || !make_weight_map(&wm, w, COUT, CIN)) return XS_CUDA_ERROR;
+    static DeviceOnce configured;
+    if (!configured.run([] { return cudaFuncSetAttribute(conv3_slab_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSlabMaxSmem)); }))
+        return XS_CUDA_ERROR;
+    const SlabArgs args{s, plan, in, bias, out, relu ? 1 : 0, error};
+    const uint64_t ctas = static_cast<uint64_t>(s.batch) * ((s.z + plan.bz - 1) / plan.bz) * ((s.y + plan.by - 1) / plan.by);
+    conv3_slab_kernel<CIN, COUT><<<static_cast<unsigned>(ctas), kSlabThreads, plan.smem, st>>>(wm, args);
+    return check_launch();
+}
+
 template <int CIN, int COUT>
 XsStatus launch_conv_forward(cudaStream_t st, const VolumeShape& s, const __nv_bfloat16* in, const __nv_bfloat16* w, const float* bias,
                              __nv_bfloat16* out, bool relu, int* error) {
     uint32_t bx, by, bz;
     if (!conv_tile(s, bx, by, bz)) return XS_INVALID_ARGUMENT;
+    // The slab wins where the 27 shifted boxes of narrow layers fill the SMs:
+    // 16 -> 16 at 64^3 26 us against 46 from the boxes, at 8 x 64^3 159
+    // against 294; 16 -> 32 at 8 x 32^3 38 against 48.  With fewer voxels a CTA
+    // has too few MMAs behind one box to wait for (16 -> 32 at 32^3 14.1 us
+    // against 11.1; by both slopes they meet near 100,000 voxels), and from 32
+    // channels on a box fills an MMA's time anyway (32 -> 16 at 8 x 32^3 52.0
+    // against 51.3, 64 -> 64 at 16^3 16.2 against 9.9).
+    if constexpr (CIN == 16) {
+        SlabPlan plan;
+        if (static_cast<uint64_t>(s.x) * s.y * s.z * s.batch >= kSlabMinVoxels && slab_plan<CIN, COUT>(s, plan))
+            return launch_conv_slab<CIN, COUT>(st, s, plan, in, w, bias, out, relu, error);
+    }
     CUtensorMap am, wm;
     if (!make_activation_map(&am, in, s, CIN, bx, by, bz) || !make_weight_map(&wm, w, COUT, CIN)) return XS_CUDA_ERROR;
     using L = ConvSmem<CIN, COUT>;
@@ -281,7 +538,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_
     uint64_t* empty = full + L::stages;
     uint64_t* accum = empty + L::stages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = static_cast<int>(tc::uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
 
     const uint32_t cx = blockIdx.x, nctas = gridDim.x;
     const uint32_t t_begin = static_cast<uint32_t>(static_cast<uint64_t>(a.tiles) * cx / nctas);
@@ -307,11 +564,12 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_
     tc::tc_fence_before();
     __syncthreads();
     tc::tc_fence_after();
-    const uint32_t tmem = *tmem_slot;
+    const uint32_t tmem = tc::uniform(*tmem_slot);
     bool ok = true;
     const uint32_t tiles_x = a.s.x / a.bx, tiles_y = a.s.y / a.by, tiles_z = a.s.z / a.bz;
 
-    if (warp == 0 && lane == 0) {
+    if (warp == 0) {
+      if (tc::elect_one()) {
         for (uint32_t i = 0; i < items; ++i) {
             const int s = static_cast<int>(i % L::stages), round = static_cast<int>(i / L::stages);
             if (i >= static_cast<uint32_t>(L::stages) && !tc::mbar_wait(&empty[s], (round - 1) & 1)) { ok = false; break; }
@@ -335,26 +593,29 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_
             }
             tc::tma_load_5d(st + L::G * L::x_tile, &dy_map, &full[s], 0, x0, y0, z, b);
         }
-    } else if (warp == 1 && lane == 0) {
+      }
+    } else if (warp == 1) {
         constexpr uint32_t idesc = tc::idesc_bf16(128, COUT, true, true);
         constexpr uint32_t a_row = CIN * 2, b_row = COUT * 2;
-        for (uint32_t i = 0; i < items; ++i) {
-            const int s = static_cast<int>(i % L::stages), round = static_cast<int>(i / L::stages);
-            if (!tc::mbar_wait(&full[s], round & 1)) { ok = false; break; }
-            tc::tc_fence_after();
-            const uint32_t gl = i % g_count;
-            const bool first_tile = (i / g_count) == 0;
-            const uint32_t xa = tc::smem_u32(smem + s * L::stage_bytes);
-            const uint32_t ya = xa + L::G * L::x_tile;
+        const uint32_t first = tc::uniform(tc::smem_u32(smem));
+        const uint64_t xs_desc = tc::smem_desc(first, L::x_tile, 8u * a_row, tc::swizzle_for_row_bytes(a_row));
+        const uint64_t dy_desc = tc::smem_desc(first + L::G * L::x_tile, L::y_padded, 8u * b_row, tc::swizzle_for_row_bytes(b_row));
+        if (tc::elect_one()) {
+            uint32_t s = 0u, round = 0u, group = 0u, accumulate = 0u;
+            for (uint32_t i = 0; i < items; ++i) {
+                if (!tc::mbar_wait(&full[s], round & 1u)) { ok = false; break; }
+                tc::tc_fence_after();
+                const uint64_t xd = xs_desc + s * (L::stage_bytes / 16u), yd = dy_desc + s * (L::stage_bytes / 16u);
+                const uint32_t d = tmem + group * COUT;
 #pragma unroll
-            for (int k = 0; k < 8; ++k) {  // 16 voxels per MMA: two 8-row atoms
-                const uint64_t ad = tc::smem_desc(xa + k * 16u * a_row, L::x_tile, 8u * a_row, tc::swizzle_for_row_bytes(a_row));
-                const uint64_t bd = tc::smem_desc(ya + k * 16u * b_row, L::y_padded, 8u * b_row, tc::swizzle_for_row_bytes(b_row));
-                tc::mma_bf16(tmem + gl * COUT, ad, bd, idesc, (!first_tile || k > 0) ? 1u : 0u);
+                for (uint32_t k = 0; k < 8u; ++k)  // 16 voxels per MMA: two 8-row atoms
+                    tc::mma_bf16(d, xd + k * a_row, yd + k * b_row, idesc, k > 0u ? 1u : accumulate);
+                tc::mma_commit(&empty[s]);
+                if (++s == static_cast<uint32_t>(L::stages)) { s = 0u; ++round; }
+                if (++group == static_cast<uint32_t>(g_count)) { group = 0u; accumulate = 1u; }
             }
-            tc::mma_commit(&empty[s]);
+            tc::mma_commit(accum);
         }
-        tc::mma_commit(accum);
     }
     __syncwarp();
     const bool got = items == 0 ? true : tc::mbar_wait(accum, 0);

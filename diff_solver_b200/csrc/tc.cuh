@@ -99,6 +99,19 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
         : "memory");
 }
 
+// True in one lane of a converged warp.  Code under it, with operands that
+// are the same in all lanes, keeps them in uniform registers: an MMA is then
+// issued every 40 cycles (128 x 16 x 16) from descriptors stepped by addition,
+// against 60 and more from one thread's own registers, where each operand is
+// moved over first.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+    return r != 0u;
+}
+// A value that is the same in all lanes, as one the compiler knows to be.
+__device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
+
 // Arrive on `bar` once all previously issued tcgen05.mma of this thread completed.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");

@@ -86,3 +86,48 @@ def test_conv_gradients_match_torch(cuda, cin, cout, shape, batch):
     assert int(err.item()) == 0
     rel = (dx.float().cpu() - xf.grad).norm() / xf.grad.norm()
     assert rel < 1e-2, (cin, cout, shape, float(rel))
+
+
+@pytest.mark.parametrize("cout,shape,batch", [
+    (16, (64, 48, 40), 1), (16, (16, 16, 98), 4), (16, (8, 48, 75), 4), (16, (32, 33 * 4, 26), 1),
+    (32, (128, 37, 22), 1), (32, (32, 32, 25), 4), (64, (64, 26, 61), 1), (64, (256, 21, 19), 1)])
+def test_conv_from_halo_slabs(cuda, cout, shape, batch):
+    """Volumes of 100,000 voxels and more with 16 input channels: ragged strips
+    of rows and layers of planes, several tiles per plane and per TMEM lane
+    block, rows longer than a tile.  Against PyTorch FP32, and, where the
+    samples by themselves take the kernel of shifted boxes, against that: the
+    two differ by the order of FP32 sums of 432 products below 1 in
+    magnitude, so by one BF16 step where a sum lies beside a rounding edge."""
+    import torch
+    from diff_solver_b200 import _native as N
+    cin = 16
+    nx, ny, nz = shape
+    assert nx * ny * nz * batch >= 100000
+    g = torch.Generator(device="cpu").manual_seed(cout + nx)
+    x = torch.randn(batch, nz, ny, nx, cin, generator=g).to(torch.bfloat16)
+    w = (torch.randn(27, cout, cin, generator=g) / (27 * cin) ** 0.5).to(torch.bfloat16)
+    bias = torch.randn(cout, generator=g).float()
+    xd, wd, bd = x.cuda(), w.cuda(), bias.cuda()
+    out = torch.full((batch, nz, ny, nx, cout), 7.0, dtype=torch.bfloat16, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+
+    def conv(samples, src, dst, relu):
+        N.check("conv", N.lib().xs_conv3d_bf16(None, samples, nx, ny, nz, cin, cout, src.data_ptr(), wd.data_ptr(), bd.data_ptr(), dst.data_ptr(),
+                                               relu, err.data_ptr()))
+
+    for relu in (0, 1):
+        conv(batch, xd, out, relu)
+        torch.cuda.synchronize()
+        assert int(err.item()) == 0
+        want = reference_conv(x.float(), w.float(), bias, relu)
+        got = out.float().cpu()
+        assert (got - want).norm() / want.norm() < 1e-2
+        # each sum is within BF16 rounding (2^-9) and FP32 accumulation of the reference
+        assert bool(((got - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all())
+    if batch > 1:
+        one = torch.empty_like(out)
+        for b in range(batch):
+            conv(1, xd[b], one[b], 1)
+        torch.cuda.synchronize()
+        assert int(err.item()) == 0
+        assert bool(((one.float() - out.float()).abs() <= 2.0 ** -7 * one.float().abs() + 1e-4).all())
