@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __gri
 // What bounds it is the rate at which one warp issues 128 x 16 x 16 MMAs, 40
 // cycles each from uniform registers: 16 -> 16 at 64^3 runs in 26 us (the
 // shifted boxes, 27 x 8.4 MB through L2: 46 to 50), 8 x 64^3 in 159 (294), of
-// which the MMAs are 130.  The unswizzled layout, 8 voxels by 16 bytes at a
+// which the MMAs are 70.  The unswizzled layout, 8 voxels by 16 bytes at a
 // time, gives the same numbers at a quarter of the operand rate: 140 cycles
 // per MMA.
 //
@@ -643,6 +643,188 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_
     if (warp == 0) tc::tmem_dealloc(tmem, 256);
 }
 
+// -------------------------------------------- weight gradient, read once
+// The same sums for up to 32 channels on either side, with every voxel brought
+// into shared memory once instead of once per tap.  A CTA walks the planes of
+// a strip of R rows; its planes of X are kept in rows of X + 1 voxels behind
+// a column of zeros, R of them, those of dY the same way with a row more on
+// either side, three deep.  In these rows two voxels that a tap pairs are the
+// same distance apart everywhere, and a pair that wraps around a row's end has
+// a zero in it, so 16 consecutive voxels of X and of dY are one K step for all
+// taps at once: the rows of the MMA are X from 128 / C_in consecutive
+// voxels on (its operand's atoms overlap, one voxel apart; the first three are
+// the taps' dx), the columns dY from three consecutive rows on (dy), one MMA
+// and one accumulator per plane of dY (dz).
+//
+// What bounds it is one warp's MMA issue, 3 per 16 voxels; the boxes per tap
+// are bound by L2 instead (27 x 67 MB at 8 x 64^3).16 -> 16 at
+// 8 x 64^3: 82.8 us (298), where the MMAs, 128 x 48 x 16 at 45 cycles, are 65.
+//
+// A voxel that is infinite or NaN also meets zeros here that no tap pairs it
+// with (a row's margin): more taps of the sums turn NaN than those it is in.
+constexpr uint64_t kWslabMinVoxels = 30000u;
+constexpr uint32_t kWsTail = 32u;  // voxels of zeros past a plane: a K step's rest and the atoms' shifts
+
+struct WslabArgs {
+    VolumeShape s;
+    uint32_t rows;      // R
+    uint32_t strips;    // per plane
+    uint32_t slots;     // planes in flight
+    uint32_t x_bytes, slot_bytes;
+    float* partial;     // [gridDim.x][27][COUT][CIN]
+    int* error;
+};
+constexpr uint32_t kWsMaxSlots = 8u;
+
+template <int CIN, int COUT>
+__global__ void __launch_bounds__(kConvThreads) conv3_wgrad_slab_kernel(const __grid_constant__ CUtensorMap x_map,
+                                                                        const __grid_constant__ CUtensorMap dy_map, WslabArgs a) {
+    constexpr uint32_t x_voxel = CIN * 2u, y_voxel = COUT * 2u, columns = 9u * COUT <= 256u ? 256u : 512u;
+    static_assert(128 / CIN >= 3 && 9 * COUT <= 512);
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
+    __shared__ uint64_t full[kWsMaxSlots], empty[kWsMaxSlots], accum[1];
+    __shared__ uint32_t tmem_slot;
+    const int warp = static_cast<int>(tc::uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
+    const uint32_t px = a.s.x + 1u, x_box = a.rows * px * x_voxel, y_box = (a.rows + 2u) * px * y_voxel;
+    const uint64_t items = static_cast<uint64_t>(a.s.batch) * a.strips * a.s.z;
+    const uint32_t first = static_cast<uint32_t>(items * blockIdx.x / gridDim.x), last = static_cast<uint32_t>(items * (blockIdx.x + 1u) / gridDim.x);
+
+    if (threadIdx.x == 0) {
+        for (uint32_t i = 0; i < a.slots; ++i) {
+            tc::mbar_init(&full[i], 1);
+            tc::mbar_init(&empty[i], 1);
+        }
+        tc::mbar_init(accum, 1);
+        tc::fence_barrier_init();
+        tc::prefetch_map(&x_map);
+        tc::prefetch_map(&dy_map);
+    }
+    if (warp == 0) {
+        tc::tmem_alloc(&tmem_slot, columns);
+        tc::tmem_relinquish();
+    }
+    for (uint32_t i = threadIdx.x; i < a.slots * kWsTail * (x_voxel + y_voxel) / 4u; i += kConvThreads) {
+        const uint32_t slot = i / (kWsTail * (x_voxel + y_voxel) / 4u), w = i % (kWsTail * (x_voxel + y_voxel) / 4u), xw = kWsTail * x_voxel / 4u;
+        unsigned char* at = smem + slot * a.slot_bytes + (w < xw ? x_box + w * 4u : a.x_bytes + y_box + (w - xw) * 4u);
+        *reinterpret_cast<uint32_t*>(at) = 0u;
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    tc::tc_fence_before();
+    __syncthreads();
+    tc::tc_fence_after();
+    const uint32_t tmem = tc::uniform(tmem_slot);
+    bool ok = true;
+
+    // Both sides walk the same stages: for the planes [z, z + n) of a strip
+    // that this CTA owns, the planes [z - 1, z + n] of dY, and from the third
+    // stage on a plane of X two behind, for which the three are there.  Stage
+    // g gives back the slot of stage g - 2.
+    if (warp == 0) {
+        if (tc::elect_one()) {
+            uint32_t slot = 0u, round = 0u;
+            for (uint32_t i = first; i < last && ok;) {
+                const uint32_t z = i % a.s.z, column = i / a.s.z, n = min(a.s.z - z, last - i);
+                const int y0 = static_cast<int>(column % a.strips * a.rows), b = static_cast<int>(column / a.strips);
+                for (uint32_t t = 0; t < n + 2u; ++t) {
+                    if (round > 0u && !tc::mbar_wait(&empty[slot], (round - 1u) & 1u)) { ok = false; break; }
+                    unsigned char* at = smem + slot * a.slot_bytes;
+                    tc::mbar_expect_tx(&full[slot], y_box + (t >= 2u ? x_box : 0u));
+                    tc::tma_load_5d(at + a.x_bytes, &dy_map, &full[slot], 0, -1, y0 - 1, static_cast<int>(z + t) - 1, b);
+                    if (t >= 2u) tc::tma_load_5d(at, &x_map, &full[slot], 0, -1, y0, static_cast<int>(z + t) - 2, b);
+                    if (++slot == a.slots) { slot = 0u; ++round; }
+                }
+                i += n;
+            }
+        }
+    } else if (warp == 1) {
+        constexpr uint32_t idesc = tc::idesc_bf16(128, 3 * COUT, true, true);
+        const uint32_t at = tc::uniform(tc::smem_u32(smem));
+        // atoms one voxel apart (X) and one row apart (dY, which starts a voxel on)
+        const uint64_t x_desc = tc::smem_desc(at, x_voxel, 8u * x_voxel, tc::swizzle_for_row_bytes(x_voxel));
+        const uint64_t y_desc = tc::smem_desc(at + a.x_bytes + y_voxel, px * y_voxel, 8u * y_voxel, tc::swizzle_for_row_bytes(y_voxel));
+        const uint32_t step = a.slot_bytes / 16u;
+        if (tc::elect_one()) {
+            uint32_t slot = 0u, round = 0u, before = 0u, two_before = 0u, accumulate = 0u, stages = 0u;
+            for (uint32_t i = first; i < last && ok;) {
+                const uint32_t z = i % a.s.z, column = i / a.s.z, n = min(a.s.z - z, last - i);
+                const uint32_t steps = (min(a.rows, a.s.y - column % a.strips * a.rows) * px + 15u) / 16u;
+                for (uint32_t t = 0; t < n + 2u; ++t, ++stages) {
+                    if (!tc::mbar_wait(&full[slot], round & 1u)) { ok = false; break; }
+                    if (t >= 2u) {
+                        tc::tc_fence_after();
+                        uint64_t xd = x_desc + slot * step, y0 = y_desc + two_before * step, y1 = y_desc + before * step, y2 = y_desc + slot * step;
+#pragma unroll 2
+                        for (uint32_t k = 0; k < steps; ++k) {
+                            tc::mma_bf16(tmem, xd, y0, idesc, accumulate);
+                            tc::mma_bf16(tmem + 3u * COUT, xd, y1, idesc, accumulate);
+                            tc::mma_bf16(tmem + 6u * COUT, xd, y2, idesc, accumulate);
+                            xd += x_voxel;  // 16 voxels, in units of 16 bytes
+                            y0 += y_voxel;
+                            y1 += y_voxel;
+                            y2 += y_voxel;
+                            accumulate = 1u;
+                        }
+                    }
+                    if (stages >= 2u) tc::mma_commit(&empty[two_before]);
+                    two_before = before;
+                    before = slot;
+                    if (++slot == a.slots) { slot = 0u; ++round; }
+                }
+                i += n;
+            }
+            tc::mma_commit(accum);
+        }
+    }
+    __syncwarp();
+    const bool got = tc::mbar_wait(accum, 0);
+    tc::tc_fence_after();
+    if (got && warp * 32 < 3 * CIN) {
+        const int m = warp * 32 + lane, dx = m / CIN, ci = m % CIN;
+        for (int d = 0; d < 9; ++d) {  // planes of dY in rising order fall to taps of falling dz, rows to dy
+            const int tap = (2 - d / 3) * 9 + (2 - d % 3) * 3 + dx;
+#pragma unroll
+            for (int c0 = 0; c0 < COUT; c0 += 16) {
+                float v[16];
+                tc::tmem_ld16(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(d * COUT + c0), v);
+                if (dx < 3) {
+                    float* dst = a.partial + ((static_cast<size_t>(blockIdx.x) * 27 + tap) * COUT + c0) * CIN + ci;
+#pragma unroll
+                    for (int q = 0; q < 16; ++q) dst[static_cast<size_t>(q) * CIN] = v[q];
+                }
+            }
+        }
+    }
+    if ((!ok || !got) && a.error) atomicExch(a.error, 1);
+    tc::tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tc::tmem_dealloc(tmem, columns);
+}
+
+// Rows of a strip: the fewest MMAs on the CTA with the most of them, with room
+// for a plane in flight beside the three in use.
+template <int CIN, int COUT>
+bool wgrad_slab_plan(const VolumeShape& s, uint32_t ctas, WslabArgs& best) {
+    const uint32_t px = s.x + 1u;
+    if (px > 256u) return false;  // the widest box of a tensor map
+    uint64_t least = 0u;
+    for (uint32_t rows = 1; rows <= std::min(s.y, 254u); ++rows) {
+        const uint32_t x_bytes = ((rows * px + kWsTail) * CIN * 2u + 1023u) / 1024u * 1024u;
+        const uint32_t slot = x_bytes + (((rows + 2u) * px + kWsTail) * COUT * 2u + 1023u) / 1024u * 1024u;
+        const uint32_t slots = std::min(kWsMaxSlots, (kSlabMaxSmem - 1024u) / slot);
+        if (slots < 4u) break;
+        const uint32_t strips = (s.y + rows - 1u) / rows;
+        const uint64_t items = static_cast<uint64_t>(s.batch) * strips * s.z, of_one = (items + ctas - 1u) / ctas;
+        // 45 cycles an MMA, a stage's hand-over, and two planes more where a strip begins
+        const uint64_t cycles = of_one * (3u * ((rows * px + 15u) / 16u) * 45u + 200u) + 2u * (of_one / s.z + 1u) * 400u;
+        if (least == 0u || cycles < least) {
+            least = cycles;
+            best = WslabArgs{s, rows, strips, slots, x_bytes, slot, nullptr, nullptr};
+        }
+    }
+    return least > 0u;
+}
+
 // dW[i] (+)= sum over CTAs of partial[cta][i], in CTA order.
 __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, uint32_t ctas, uint32_t count, float* __restrict__ dw, int accumulate) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -676,10 +858,33 @@ XsStatus launch_wgrad(cudaStream_t st, const VolumeShape& s, const __nv_bfloat16
         return XS_CUDA_ERROR;
     const uint32_t tiles = static_cast<uint32_t>(static_cast<uint64_t>(s.batch) * (s.z / bz) * (s.y / by) * (s.x / bx));
     const uint32_t ctas = wgrad_ctas(s);
+    const uint32_t count = 27u * CIN * COUT;
+    if constexpr (CIN <= 32 && COUT <= 32) {
+        // 16 -> 16 at 8 x 64^3 82.8 us against 298 from the boxes, at 64^3 22.9
+        // against 48.0, at 32^3 14.5 against 16.5, where a CTA has 6 planes
+        // and two thirds of the time is the launches and the wait for its
+        // first three loads; 32 -> 32 at 8 x 32^3 20.3 against 55.
+        WslabArgs slab{};
+        if (static_cast<uint64_t>(s.x) * s.y * s.z * s.batch >= kWslabMinVoxels && wgrad_slab_plan<CIN, COUT>(s, ctas, slab)) {
+            if (!make_activation_map(&xm, x, s, CIN, s.x + 1u, slab.rows, 1) || !make_activation_map(&ym, dy, s, COUT, s.x + 1u, slab.rows + 2u, 1))
+                return XS_CUDA_ERROR;
+            static DeviceOnce slab_configured;
+            if (!slab_configured.run([] {
+                    return cudaFuncSetAttribute(conv3_wgrad_slab_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSlabMaxSmem));
+                }))
+                return XS_CUDA_ERROR;
+            slab.partial = partial;
+            slab.error = error;
+            const uint32_t planes = s.batch * slab.strips * s.z, slab_ctas = std::min(ctas, planes);
+            conv3_wgrad_slab_kernel<CIN, COUT><<<slab_ctas, kConvThreads, 1024u + slab.slots * slab.slot_bytes, st>>>(xm, ym, slab);
+            if (check_launch() != XS_OK) return XS_CUDA_ERROR;
+            wgrad_reduce_kernel<<<(count + 255) / 256, 256, 0, st>>>(partial, slab_ctas, count, dw, accumulate ? 1 : 0);
+            return check_launch();
+        }
+    }
     WgradArgs args{s, bx, by, bz, tiles, partial, error};
     conv3_wgrad_kernel<CIN, COUT><<<dim3(ctas, L::sets), kConvThreads, L::total, st>>>(xm, ym, args);
     if (check_launch() != XS_OK) return XS_CUDA_ERROR;
-    const uint32_t count = 27u * CIN * COUT;
     wgrad_reduce_kernel<<<(count + 255) / 256, 256, 0, st>>>(partial, ctas, count, dw, accumulate ? 1 : 0);
     return check_launch();
 }

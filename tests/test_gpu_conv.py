@@ -131,3 +131,35 @@ def test_conv_from_halo_slabs(cuda, cout, shape, batch):
         torch.cuda.synchronize()
         assert int(err.item()) == 0
         assert bool(((one.float() - out.float()).abs() <= 2.0 ** -7 * one.float().abs() + 1e-4).all())
+
+
+@pytest.mark.parametrize("cin,cout,shape,batch", [
+    (16, 16, (64, 48, 40), 1), (16, 16, (16, 24, 131), 2), (16, 32, (32, 36, 30), 3), (32, 16, (64, 26, 31), 2), (32, 32, (128, 37, 22), 1),
+    (16, 16, (4, 64, 100), 4), (32, 32, (8, 48, 140), 2), (16, 16, (256, 21, 19), 1), (16, 16, (128, 800, 1), 1),
+    (16, 16, (16, 24, 79), 1), (32, 32, (2, 128, 120), 1)])
+def test_conv_weight_gradient_from_slabs(cuda, cin, cout, shape, batch):
+    """Volumes of 30,000 voxels and more with up to 32 channels: ragged
+    strips, CTAs that begin in the middle of a strip, rows too long for the
+    slab (256).  Against FP64 sums of the same BF16 products, exact in FP32:
+    the accumulation of n products in FP32, random in sign, is within a few
+    sqrt(n) roundings; 1e-5 of the norm holds with a margin of ten."""
+    import torch
+    from diff_solver_b200 import _native as N
+    L = N.lib()
+    nx, ny, nz = shape
+    assert nx * ny * nz * batch >= 30000
+    g = torch.Generator(device="cpu").manual_seed(3 * cin + cout + nx)
+    x = torch.randn(batch, nz, ny, nx, cin, generator=g).to(torch.bfloat16).cuda()
+    dy = torch.randn(batch, nz, ny, nx, cout, generator=g).to(torch.bfloat16).cuda()
+    padded = torch.nn.functional.pad(x.double(), (0, 0, 1, 1, 1, 1, 1, 1))
+    want = torch.stack([torch.einsum("bzyxi,bzyxo->oi", padded[:, dz:dz + nz, ddy:ddy + ny, dx:dx + nx], dy.double())
+                        for dz, ddy, dx in itertools.product(range(3), repeat=3)])
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    scratch = torch.full((L.xs_conv3d_weight_grad_scratch_floats(batch, nx, ny, nz, cin, cout),), float("nan"), device="cuda")
+    dw = torch.full((27, cout, cin), 2.0, dtype=torch.float32, device="cuda")
+    for accumulate in (0, 1):
+        N.check("wgrad", L.xs_conv3d_weight_grad_bf16(None, batch, nx, ny, nz, cin, cout, x.data_ptr(), dy.data_ptr(), scratch.data_ptr(),
+                                                      dw.data_ptr(), accumulate, err.data_ptr()))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    assert float((dw.double() / 2.0 - want).norm() / want.norm()) < 1e-5
