@@ -122,38 +122,56 @@ __global__ void integrate_vjp_open_cells_kernel(Grid g, XsAdjointVector oa, XsAd
     }
 }
 
-// Shared tail of both advection adjoints (operators.cu:426-438, 548-560):
-// adjoint of value1 through the final position, midpoint sample gradients,
-// then of value0 at the start.
-__device__ __forceinline__ void trace_adjoint(const Vec3& start, const Vec3& mid, const Trace& t, const Vec3& src_gradient, double o,
-                                              const XsVector& u, const Grid& g, const XsVelocityBoundary& vb, const XsAdjointVector& ua) {
-    const double v1x = -static_cast<double>(t.derivative.x * g.dt * src_gradient.x) * o;
-    const double v1y = -static_cast<double>(t.derivative.y * g.dt * src_gradient.y) * o;
-    const double v1z = -static_cast<double>(t.derivative.z * g.dt * src_gradient.z) * o;
-    const Sample m0 = sample_face<true>(u.x, 0, mid, g, vb);
-    const Sample m1 = sample_face<true>(u.y, 1, mid, g, vb);
-    const Sample m2 = sample_face<true>(u.z, 2, mid, g, vb);
-    scatter_face(ua.x, 0, mid, v1x, g, vb);
-    scatter_face(ua.y, 1, mid, v1y, g, vb);
-    scatter_face(ua.z, 2, mid, v1z, g, vb);
-    const double mx = m0.gradient.x * v1x + m1.gradient.x * v1y + m2.gradient.x * v1z;
-    const double my = m0.gradient.y * v1x + m1.gradient.y * v1y + m2.gradient.y * v1z;
-    const double mz = m0.gradient.z * v1x + m1.gradient.z * v1y + m2.gradient.z * v1z;
+// Adjoint of the velocity at the midpoint through one sample at the end
+// position (operators.cu:426-428, 548-550), added to v1: what follows is linear
+// in it, so samples that share a trace (density and temperature) also share
+// the scatters.
+struct MidAdjoint {
+    double x, y, z;
+};
+__device__ __forceinline__ void add_end_adjoint(MidAdjoint& v1, const Vec3& derivative, float dt, const Vec3& src_gradient, double o) {
+    v1.x -= static_cast<double>(derivative.x * dt * src_gradient.x) * o;
+    v1.y -= static_cast<double>(derivative.y * dt * src_gradient.y) * o;
+    v1.z -= static_cast<double>(derivative.z * dt * src_gradient.z) * o;
+}
+
+// Shared tail of both advection adjoints (operators.cu:429-438, 551-560): v1
+// through the midpoint sample gradients m, then of value0 at the start.
+__device__ __forceinline__ void trace_adjoint(const Vec3& start, const Vec3& mid, const Sample (&m)[3], const MidAdjoint& v1, const Grid& g,
+                                              const XsVelocityBoundary& vb, const XsAdjointVector& ua) {
+    scatter_face(ua.x, 0, mid, v1.x, g, vb);
+    scatter_face(ua.y, 1, mid, v1.y, g, vb);
+    scatter_face(ua.z, 2, mid, v1.z, g, vb);
+    const double mx = m[0].gradient.x * v1.x + m[1].gradient.x * v1.y + m[2].gradient.x * v1.z;
+    const double my = m[0].gradient.y * v1.x + m[1].gradient.y * v1.y + m[2].gradient.y * v1.z;
+    const double mz = m[0].gradient.z * v1.x + m[1].gradient.z * v1.y + m[2].gradient.z * v1.z;
     scatter_face(ua.x, 0, start, -0.5 * static_cast<double>(g.dt) * mx, g, vb);
     scatter_face(ua.y, 1, start, -0.5 * static_cast<double>(g.dt) * my, g, vb);
     scatter_face(ua.z, 2, start, -0.5 * static_cast<double>(g.dt) * mz, g, vb);
+}
+
+// The RK2 trace with its midpoint and the samples there.
+__device__ __forceinline__ Trace trace_with_samples(const Vec3& s, const XsVector& u, const uint32_t* __restrict__ mask, const Grid& g,
+                                                    const XsVelocityBoundary& vb, Vec3& mid, Sample (&m)[3]) {
+    mid = trace_midpoint(s, sample_velocity(u.x, u.y, u.z, s, g, vb), g);
+    m[0] = sample_face<true>(u.x, 0, mid, g, vb);
+    m[1] = sample_face<true>(u.y, 1, mid, g, vb);
+    m[2] = sample_face<true>(u.z, 2, mid, g, vb);
+    return trace_end(s, Vec3{m[0].value, m[1].value, m[2].value}, mask, g, vb);
 }
 
 // operators.cu:415-439, one face (general form: colliders, any spacing).
 __device__ __forceinline__ void advect_velocity_vjp_face(int a, int x, int y, int z, double o, const Grid& g, const uint32_t* __restrict__ mask,
                                                          const XsVector& u, const XsVelocityBoundary& vb, const XsAdjointVector& ua) {
     const Vec3 s = face_position(a, x, y, z, g);
-    const Vec3 v0 = sample_velocity(u.x, u.y, u.z, s, g, vb);
-    const Vec3 mid{s.x - 0.5f * g.dt * v0.x, s.y - 0.5f * g.dt * v0.y, s.z - 0.5f * g.dt * v0.z};
-    const Trace t = trace_rk2(s, u.x, u.y, u.z, mask, g, vb);
+    Vec3 mid;
+    Sample m[3];
+    const Trace t = trace_with_samples(s, u, mask, g, vb, mid, m);
     const Sample src = sample_face<true>(component<const float>(u.x, u.y, u.z, a), a, t.position, g, vb);
     scatter_face(component<double>(ua.x, ua.y, ua.z, a), a, t.position, o, g, vb);
-    trace_adjoint(s, mid, t, src.gradient, o, u, g, vb, ua);
+    MidAdjoint v1{0.0, 0.0, 0.0};
+    add_end_adjoint(v1, t.derivative, g.dt, src.gradient, o);
+    trace_adjoint(s, mid, m, v1, g, vb, ua);
 }
 
 // operators.cu:415-439 for all three components in one launch.
@@ -177,7 +195,8 @@ __global__ void advect_velocity_vjp_kernel(const __grid_constant__ Grid g, uint6
 // gathers goes to FP64 box accumulators in shared memory, and each touched
 // box node is added to global memory once at the end (instead of 56 global
 // atomics per face).  The same products as the general kernels; only the
-// order of the FP64 additions differs.
+// order of the FP64 additions differs.  Density and temperature share the
+// scatters behind their common trace: 461 us at 128^3, 595 with one each.
 // Halo 1: the box holds every stencil of traces shorter than half a cell per
 // step (longer ones scatter to global memory); the smaller boxes give five
 // velocity-adjoint CTAs per SM (96 registers: 6.49 against 6.88 ms at 256^3
@@ -186,24 +205,20 @@ using AdjointTile = tile::Shape<32, 4, 4, 1>;
 constexpr size_t kVelocityVjpSmem = 3 * AdjointTile::kNodes * (sizeof(double) + sizeof(float));
 constexpr size_t kScalarVjpSmem = 5 * AdjointTile::kNodes * (sizeof(double) + sizeof(float));
 
-// The trace adjoint of one sample at the trace end (operators.cu:426-438):
-// through the end position to the midpoint samples (their gradients m), and
+// The trace adjoint of the samples at the trace end (operators.cu:426-438)
+// from their sum v1: through the midpoint samples (their gradients m), and
 // through the midpoint to the start (exact start weights).  A is the face
 // component at run time (a cell centre for the scalar adjoints: cell).
-__device__ __forceinline__ void staged_trace_adjoint(int A, const Vec3& mid, const Sample (&m)[3], const Vec3& der, const Vec3& src_gradient,
-                                                     double o, int li, double* const (&acc)[3], const tile::Origin& org,
-                                                     const tile::TileConsts& k, const Grid& g, const XsVelocityBoundary& vb,
-                                                     const XsAdjointVector& ua, bool cell) {
+__device__ __forceinline__ void staged_trace_adjoint(int A, const Vec3& mid, const Sample (&m)[3], const MidAdjoint& v1, int li,
+                                                     double* const (&acc)[3], const tile::Origin& org, const tile::TileConsts& k, const Grid& g,
+                                                     const XsVelocityBoundary& vb, const XsAdjointVector& ua, bool cell) {
     using S = AdjointTile;
-    const double v1x = -static_cast<double>(der.x * g.dt * src_gradient.x) * o;
-    const double v1y = -static_cast<double>(der.y * g.dt * src_gradient.y) * o;
-    const double v1z = -static_cast<double>(der.z * g.dt * src_gradient.z) * o;
-    tile::staged_face_scatter<S, 0>(acc[0], ua.x, mid, v1x, org, k, g, vb);
-    tile::staged_face_scatter<S, 1>(acc[1], ua.y, mid, v1y, org, k, g, vb);
-    tile::staged_face_scatter<S, 2>(acc[2], ua.z, mid, v1z, org, k, g, vb);
-    const double mx = m[0].gradient.x * v1x + m[1].gradient.x * v1y + m[2].gradient.x * v1z;
-    const double my = m[0].gradient.y * v1x + m[1].gradient.y * v1y + m[2].gradient.y * v1z;
-    const double mz = m[0].gradient.z * v1x + m[1].gradient.z * v1y + m[2].gradient.z * v1z;
+    tile::staged_face_scatter<S, 0>(acc[0], ua.x, mid, v1.x, org, k, g, vb);
+    tile::staged_face_scatter<S, 1>(acc[1], ua.y, mid, v1.y, org, k, g, vb);
+    tile::staged_face_scatter<S, 2>(acc[2], ua.z, mid, v1.z, org, k, g, vb);
+    const double mx = m[0].gradient.x * v1.x + m[1].gradient.x * v1.y + m[2].gradient.x * v1.z;
+    const double my = m[0].gradient.y * v1.x + m[1].gradient.y * v1.y + m[2].gradient.y * v1.z;
+    const double mz = m[0].gradient.z * v1.x + m[1].gradient.z * v1.y + m[2].gradient.z * v1.z;
     const double h = -0.5 * static_cast<double>(g.dt);
     if (cell) {
         tile::cell_start_scatter<S, 0>(acc[0], li, h * mx);
@@ -247,7 +262,9 @@ __device__ __forceinline__ void advect_velocity_vjp_tile_face(int A, int x, int 
     const Vec3 end = staged_trace_with_samples(sv, s, tile::face_start_velocity_rt<S>(sv, li, A), org, k, g, vb, mid, m, der);
     const Sample src = tile::staged_face_rt<S>(sv.s[A], component<const float>(sv.u.x, sv.u.y, sv.u.z, A), A, end, org, k, g, vb);
     tile::staged_face_scatter_rt<S>(acc[A], component<double>(ua.x, ua.y, ua.z, A), A, end, o, org, k, g, vb);
-    staged_trace_adjoint(A, mid, m, der, src.gradient, o, li, acc, org, k, g, vb, ua, false);
+    MidAdjoint v1{0.0, 0.0, 0.0};
+    add_end_adjoint(v1, der, g.dt, src.gradient, o);
+    staged_trace_adjoint(A, mid, m, v1, li, acc, org, k, g, vb, ua, false);
 }
 
 __global__ void __launch_bounds__(AdjointTile::kThreads, 5) advect_velocity_vjp_tile_kernel(const __grid_constant__ Grid g, XsVector u, const __grid_constant__ XsVelocityBoundary vb,
@@ -351,14 +368,18 @@ __global__ void __launch_bounds__(AdjointTile::kThreads, 3) advect_scalar_vjp_ti
             Vec3 mid, der;
             Sample m[3];
             const Vec3 end = staged_trace_with_samples(sv, s, tile::cell_start_velocity<S>(sv, li), org, k, g, vb, mid, m, der);
-            const Sample smp = tile::staged_scalar<S, true>(box + 3 * S::kNodes, src, end, org, k, g, sb);
-            tile::staged_scalar_scatter<S>(sacc[0], sa, end, o1, org, k, g, sb);
-            if (o1 != 0.0) staged_trace_adjoint(0, mid, m, der, smp.gradient, o1, li, acc, org, k, g, vb, ua, true);
-            if (two && o2 != 0.0) {
-                const Sample smp2 = tile::staged_scalar<S, true>(box + 4 * S::kNodes, src2, end, org, k, g, sb2);
-                tile::staged_scalar_scatter<S>(sacc[1], sa2, end, o2, org, k, g, sb2);
-                staged_trace_adjoint(0, mid, m, der, smp2.gradient, o2, li, acc, org, k, g, vb, ua, true);
+            MidAdjoint v1{0.0, 0.0, 0.0};
+            if (o1 != 0.0) {
+                const Sample smp = tile::staged_scalar<S, true>(box + 3 * S::kNodes, src, end, org, k, g, sb);
+                tile::staged_scalar_scatter<S>(sacc[0], sa, end, o1, org, k, g, sb);
+                add_end_adjoint(v1, der, g.dt, smp.gradient, o1);
             }
+            if (o2 != 0.0) {
+                const Sample smp = tile::staged_scalar<S, true>(box + 4 * S::kNodes, src2, end, org, k, g, sb2);
+                tile::staged_scalar_scatter<S>(sacc[1], sa2, end, o2, org, k, g, sb2);
+                add_end_adjoint(v1, der, g.dt, smp.gradient, o2);
+            }
+            staged_trace_adjoint(0, mid, m, v1, li, acc, org, k, g, vb, ua, true);
         }
     }
     __syncthreads();
@@ -383,17 +404,21 @@ __global__ void advect_scalar_vjp_kernel(const __grid_constant__ Grid g, const u
     int x, y, z;
     decode(i, g.nx, g.ny, x, y, z);
     const Vec3 s = cell_position(x, y, z, g);
-    const Vec3 v0 = sample_velocity(u.x, u.y, u.z, s, g, vb);
-    const Vec3 mid{s.x - 0.5f * g.dt * v0.x, s.y - 0.5f * g.dt * v0.y, s.z - 0.5f * g.dt * v0.z};
-    const Trace t = trace_rk2(s, u.x, u.y, u.z, mask, g, vb);
-    const Sample smp = sample_scalar<true>(src, t.position, g, sb);
-    scatter_scalar(sa, t.position, o1, g, sb);
-    trace_adjoint(s, mid, t, smp.gradient, o1, u, g, vb, ua);
-    if (oa2 && o2 != 0.0) {
-        const Sample smp2 = sample_scalar<true>(src2, t.position, g, sb2);
-        scatter_scalar(sa2, t.position, o2, g, sb2);
-        trace_adjoint(s, mid, t, smp2.gradient, o2, u, g, vb, ua);
+    Vec3 mid;
+    Sample m[3];
+    const Trace t = trace_with_samples(s, u, mask, g, vb, mid, m);
+    MidAdjoint v1{0.0, 0.0, 0.0};
+    if (o1 != 0.0) {
+        const Sample smp = sample_scalar<true>(src, t.position, g, sb);
+        scatter_scalar(sa, t.position, o1, g, sb);
+        add_end_adjoint(v1, t.derivative, g.dt, smp.gradient, o1);
     }
+    if (o2 != 0.0) {
+        const Sample smp = sample_scalar<true>(src2, t.position, g, sb2);
+        scatter_scalar(sa2, t.position, o2, g, sb2);
+        add_end_adjoint(v1, t.derivative, g.dt, smp.gradient, o2);
+    }
+    trace_adjoint(s, mid, m, v1, g, vb, ua);
 }
 
 // ---------------------------------------------------------------- constrain

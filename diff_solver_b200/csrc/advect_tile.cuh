@@ -84,10 +84,9 @@ __device__ __forceinline__ void stage_wait() { asm volatile("cp.async.wait_all;"
 // Stages face component A over the box: one warp per box row (x-contiguous,
 // coalesced), two passes for the row's SX nodes.  A box inside the array is
 // copied asynchronously by a short unrolled loop; a box that crosses the
-// domain edge (rolled loop, one copy of the boundary logic) copies its
-// in-array nodes asynchronously and applies the boundary rules to the nodes
-// beyond the edge only.  The caller runs stage_wait() and __syncthreads()
-// before reading the box.
+// domain edge applies the boundary rules per axis (a lane's x once, y and z
+// per row): a node takes a fixed value or is copied from its partner.  The
+// caller runs stage_wait() and __syncthreads() before reading the box.
 template <class S, int A>
 __device__ __forceinline__ void stage_face(float* __restrict__ s, const float* __restrict__ v, const Origin& o, const Grid& g,
                                            const XsVelocityBoundary& b) {
@@ -108,20 +107,20 @@ __device__ __forceinline__ void stage_face(float* __restrict__ s, const float* _
         }
         return;
     }
+    const AxisNode nx[2] = {face_axis_node(0, o.x + lane, ex, g.nx, A, b), face_axis_node(0, o.x + lane + 32, ex, g.nx, A, b)};
 #pragma unroll 1
     for (int row = warp; row < S::kRows; row += S::TY) {
-        const int y = o.y + row % S::SY, z = o.z + row / S::SY;
-        const bool row_in = static_cast<unsigned>(y) < static_cast<unsigned>(ly) && static_cast<unsigned>(z) < static_cast<unsigned>(lz);
+        const AxisNode ny = face_axis_node(1, o.y + row % S::SY, ey, g.ny, A, b), nz = face_axis_node(2, o.z + row / S::SY, ez, g.nz, A, b);
+        const float* src = v + index32(0, ny.at, nz.at, ex, ey);
         float* dst = s + row * S::SX;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int bx = lane + 32 * half;
             if (half == 1 && bx >= S::SX) break;
-            const int x = o.x + bx;
-            if (row_in && static_cast<unsigned>(x) < static_cast<unsigned>(lx))
-                cp_async4(dst + bx, v + index32(x, y, z, ex, ey));
+            if (nx[half].fixed || ny.fixed || nz.fixed)
+                dst[bx] = nx[half].fixed ? nx[half].value : (ny.fixed ? ny.value : nz.value);
             else
-                dst[bx] = load_face(v, A, x, y, z, g, b);
+                cp_async4(dst + bx, src + nx[half].at);
         }
     }
 }
@@ -143,20 +142,20 @@ __device__ __forceinline__ void stage_cells(float* __restrict__ s, const float* 
         }
         return;
     }
+    const AxisNode nx[2] = {cell_axis_node(0, o.x + lane, g.nx, b), cell_axis_node(0, o.x + lane + 32, g.nx, b)};
 #pragma unroll 1
     for (int row = warp; row < S::kRows; row += S::TY) {
-        const int y = o.y + row % S::SY, z = o.z + row / S::SY;
-        const bool row_in = static_cast<unsigned>(y) < static_cast<unsigned>(g.ny) && static_cast<unsigned>(z) < static_cast<unsigned>(g.nz);
+        const AxisNode ny = cell_axis_node(1, o.y + row % S::SY, g.ny, b), nz = cell_axis_node(2, o.z + row / S::SY, g.nz, b);
+        const float* src = v + index32(0, ny.at, nz.at, g.nx, g.ny);
         float* dst = s + row * S::SX;
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int bx = lane + 32 * half;
             if (half == 1 && bx >= S::SX) break;
-            const int x = o.x + bx;
-            if (row_in && static_cast<unsigned>(x) < static_cast<unsigned>(g.nx))
-                cp_async4(dst + bx, v + index32(x, y, z, g.nx, g.ny));
+            if (nx[half].fixed || ny.fixed || nz.fixed)
+                dst[bx] = nx[half].fixed ? nx[half].value : (ny.fixed ? ny.value : nz.value);
             else
-                dst[bx] = load_scalar(v, x, y, z, g, b);
+                cp_async4(dst + bx, src + nx[half].at);
         }
     }
 }

@@ -53,27 +53,31 @@ __global__ void buoyancy_jvp_kernel(Grid g, const uint32_t* __restrict__ mask, c
     out.z[i] = acc_t.z[i];
 }
 
-// Tangent of the RK2 trace: returns the tangent of the final position
-// (operators.cu:398-410 / 520-532).
-__device__ __forceinline__ Vec3 trace_tangent(const Vec3& s, const XsVector& u, const XsVector& ut, const Trace& t, const Grid& g,
-                                              const XsVelocityBoundary& vb, const XsVelocityBoundary& tvb) {
+// The RK2 trace and the tangent of its final position (operators.cu:398-410 /
+// 520-532), from one set of samples.  tvb is vb with zero values: a kernel
+// parameter, since a copy made in the kernel and passed on to the edge samples
+// by reference lives in local memory.
+__device__ __forceinline__ Trace trace_with_tangent(const Vec3& s, const XsVector& u, const XsVector& ut, const uint32_t* mask, const Grid& g,
+                                                    const XsVelocityBoundary& vb, const XsVelocityBoundary& tvb, Vec3& tangent) {
     const Vec3 v0 = sample_velocity(u.x, u.y, u.z, s, g, vb);
     const Vec3 t0 = sample_velocity(ut.x, ut.y, ut.z, s, g, tvb);
-    const Vec3 mid{s.x - 0.5f * g.dt * v0.x, s.y - 0.5f * g.dt * v0.y, s.z - 0.5f * g.dt * v0.z};
+    const Vec3 mid = trace_midpoint(s, v0, g);
     const Vec3 midt{-0.5f * g.dt * t0.x, -0.5f * g.dt * t0.y, -0.5f * g.dt * t0.z};
     const Sample a = sample_face<true>(u.x, 0, mid, g, vb);
     const Sample b = sample_face<true>(u.y, 1, mid, g, vb);
     const Sample c = sample_face<true>(u.z, 2, mid, g, vb);
+    const Trace t = trace_end(s, Vec3{a.value, b.value, c.value}, mask, g, vb);
     const Vec3 st = sample_velocity(ut.x, ut.y, ut.z, mid, g, tvb);
     const Vec3 v1t{st.x + a.gradient.x * midt.x + a.gradient.y * midt.y + a.gradient.z * midt.z,
                    st.y + b.gradient.x * midt.x + b.gradient.y * midt.y + b.gradient.z * midt.z,
                    st.z + c.gradient.x * midt.x + c.gradient.y * midt.y + c.gradient.z * midt.z};
-    return Vec3{-t.derivative.x * g.dt * v1t.x, -t.derivative.y * g.dt * v1t.y, -t.derivative.z * g.dt * v1t.z};
+    tangent = Vec3{-t.derivative.x * g.dt * v1t.x, -t.derivative.y * g.dt * v1t.y, -t.derivative.z * g.dt * v1t.z};
+    return t;
 }
 
 // operators.cu:390-413 for all three components in one launch.
 __global__ void advect_velocity_jvp_kernel(const __grid_constant__ Grid g, uint64_t f0, uint64_t f1, uint64_t f2, const uint32_t* __restrict__ mask, XsVector u,
-                                           XsVector ut, const __grid_constant__ XsVelocityBoundary vb, XsVector out) {
+                                           XsVector ut, const __grid_constant__ XsVelocityBoundary vb, const __grid_constant__ XsVelocityBoundary tvb, XsVector out) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= f0 + f1 + f2) return;
     int a;
@@ -81,10 +85,9 @@ __global__ void advect_velocity_jvp_kernel(const __grid_constant__ Grid g, uint6
     if (i < f0) { a = 0; local = i; } else if (i < f0 + f1) { a = 1; local = i - f0; } else { a = 2; local = i - f0 - f1; }
     int x, y, z;
     decode(local, extent(g, a, 0), extent(g, a, 1), x, y, z);
-    const XsVelocityBoundary tvb = zero_values(vb);
     const Vec3 s = face_position(a, x, y, z, g);
-    const Trace t = trace_rk2(s, u.x, u.y, u.z, mask, g, vb);
-    const Vec3 pt = trace_tangent(s, u, ut, t, g, vb, tvb);
+    Vec3 pt;
+    const Trace t = trace_with_tangent(s, u, ut, mask, g, vb, tvb, pt);
     const Sample src = sample_face<true>(component<const float>(u.x, u.y, u.z, a), a, t.position, g, vb);
     component<float>(out.x, out.y, out.z, a)[local] =
         sample_face<false>(component<const float>(ut.x, ut.y, ut.z, a), a, t.position, g, tvb).value + src.gradient.x * pt.x +
@@ -95,7 +98,9 @@ __global__ void advect_velocity_jvp_kernel(const __grid_constant__ Grid g, uint6
 __global__ void advect_scalar_jvp_kernel(const __grid_constant__ Grid g, const uint32_t* __restrict__ mask, const float* __restrict__ src,
                                          const float* __restrict__ src_t, const __grid_constant__ XsScalarBoundary sb, float* __restrict__ out,
                                          const float* __restrict__ src2, const float* __restrict__ src2_t, const __grid_constant__ XsScalarBoundary sb2,
-                                         float* __restrict__ out2, XsVector u, XsVector ut, const __grid_constant__ XsVelocityBoundary vb) {
+                                         float* __restrict__ out2, XsVector u, XsVector ut, const __grid_constant__ XsVelocityBoundary vb,
+                                         const __grid_constant__ XsVelocityBoundary tvb, const __grid_constant__ XsScalarBoundary tsb,
+                                         const __grid_constant__ XsScalarBoundary tsb2) {
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= cell_count(g)) return;
     if (is_solid(mask, i)) {
@@ -105,15 +110,14 @@ __global__ void advect_scalar_jvp_kernel(const __grid_constant__ Grid g, const u
     }
     int x, y, z;
     decode(i, g.nx, g.ny, x, y, z);
-    const XsVelocityBoundary tvb = zero_values(vb);
     const Vec3 s = cell_position(x, y, z, g);
-    const Trace t = trace_rk2(s, u.x, u.y, u.z, mask, g, vb);
-    const Vec3 pt = trace_tangent(s, u, ut, t, g, vb, tvb);
+    Vec3 pt;
+    const Trace t = trace_with_tangent(s, u, ut, mask, g, vb, tvb, pt);
     const Sample a = sample_scalar<true>(src, t.position, g, sb);
-    out[i] = sample_scalar<false>(src_t, t.position, g, zero_values(sb)).value + a.gradient.x * pt.x + a.gradient.y * pt.y + a.gradient.z * pt.z;
+    out[i] = sample_scalar<false>(src_t, t.position, g, tsb).value + a.gradient.x * pt.x + a.gradient.y * pt.y + a.gradient.z * pt.z;
     if (out2) {
         const Sample b = sample_scalar<true>(src2, t.position, g, sb2);
-        out2[i] = sample_scalar<false>(src2_t, t.position, g, zero_values(sb2)).value + b.gradient.x * pt.x + b.gradient.y * pt.y +
+        out2[i] = sample_scalar<false>(src2_t, t.position, g, tsb2).value + b.gradient.x * pt.x + b.gradient.y * pt.y +
                   b.gradient.z * pt.z;
     }
 }
@@ -139,7 +143,7 @@ XsStatus launch_buoyancy_jvp(cudaStream_t st, const Grid& g, const uint32_t* mas
 XsStatus launch_advect_velocity_jvp(cudaStream_t st, const Grid& g, const uint32_t* mask, const XsVector& u, const XsVector& ut,
                                     const XsVelocityBoundary& vb, const XsVector& out) {
     const uint64_t f0 = face_count(g, 0), f1 = face_count(g, 1), f2 = face_count(g, 2);
-    advect_velocity_jvp_kernel<<<blocks_for(f0 + f1 + f2), kBlock, 0, st>>>(g, f0, f1, f2, mask, u, ut, vb, out);
+    advect_velocity_jvp_kernel<<<blocks_for(f0 + f1 + f2), kBlock, 0, st>>>(g, f0, f1, f2, mask, u, ut, vb, zero_values(vb), out);
     return check_launch();
 }
 
@@ -147,7 +151,8 @@ XsStatus launch_advect_scalar_jvp(cudaStream_t st, const Grid& g, const uint32_t
                                   const XsScalarBoundary& sb, float* out, const float* src2, const float* src2_t,
                                   const XsScalarBoundary& sb2, float* out2, const XsVector& u, const XsVector& ut,
                                   const XsVelocityBoundary& vb) {
-    advect_scalar_jvp_kernel<<<blocks_for(cell_count(g)), kBlock, 0, st>>>(g, mask, src, src_t, sb, out, src2, src2_t, sb2, out2, u, ut, vb);
+    advect_scalar_jvp_kernel<<<blocks_for(cell_count(g)), kBlock, 0, st>>>(g, mask, src, src_t, sb, out, src2, src2_t, sb2, out2, u, ut, vb, zero_values(vb),
+                                                                        zero_values(sb), zero_values(sb2));
     return check_launch();
 }
 
