@@ -209,10 +209,9 @@ __device__ __forceinline__ void grid_coordinates(const Vec3& p, float h, int axi
 
 // True when the 2x2x2 stencil with lower corner (x0, y0, z0) lies inside an
 // array whose rows run to lx, ly, lz with no boundary rule involved: then
-// load_scalar / load_face return plain array elements, and the stencil is
-// read with 32-bit offsets and no per-node boundary logic (the same values,
-// so the same results).  lx etc. are the array extents, or the wrap period
-// on a periodic axis.
+// the nodes are plain array elements, and the stencil is read with 32-bit
+// offsets and no boundary logic (the same values, so the same results).  lx
+// etc. are the array extents, or the wrap period on a periodic axis.
 __device__ __forceinline__ bool interior_stencil(int x0, int y0, int z0, int lx, int ly, int lz) {
     return static_cast<unsigned>(x0) + 1u < static_cast<unsigned>(lx) && static_cast<unsigned>(y0) + 1u < static_cast<unsigned>(ly) &&
            static_cast<unsigned>(z0) + 1u < static_cast<unsigned>(lz) && x0 >= 0 && y0 >= 0 && z0 >= 0;
