@@ -940,10 +940,9 @@ def main():
                           f"rest (spin-up {args.spinup} steps), Jacobi-PCG to rel. residual 1e-6",
               "grid": list(args.shape), "cells": n, "faces": faces, "dt": "0.5 dx", "steps_per_replica": args.steps,
               "spinup_steps": args.spinup,
-              "warm_start": f"Galerkin start over the last {HISTORY} solutions"
-                            + (f", 6 Jacobi sweeps and a step along the coarse-grid correction (grid coarsened x{args.coarsening}, "
-                               f"solved exactly by the eigenbases of its separable operator; adjoint solves: three such rounds)"
-                               if args.coarsening else "")
+              "warm_start": ("direct solve on the fluid grid by the folded eigenbases of its separable operator, FP32, and a second "
+                             "one on the FP64 residual (adjoint solves likewise)" if args.coarsening else
+                             f"Galerkin start over the last {HISTORY} solutions")
                             + ("" if args.no_learned else
                                f", step along the U-Net correction (network trained at 128^3, applied on the grid restricted "
                                f"x{args.network_factor})"),
