@@ -221,8 +221,8 @@ __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __gri
 // holds all 27 of the narrowest layers.
 //
 // What bounds it is the rate at which one warp issues 128 x 16 x 16 MMAs, 40
-// cycles each from uniform registers: 16 -> 16 at 64^3 runs in 26 us (the
-// shifted boxes, 27 x 8.4 MB through L2: 46 to 50), 8 x 64^3 in 159 (294), of
+// cycles each from uniform registers: 16 -> 16 at 64^3 runs in 23 us (the
+// shifted boxes, 27 x 8.4 MB through L2: 46 to 50), 8 x 64^3 in 153 (294), of
 // which the MMAs are 70.  The unswizzled layout, 8 voxels by 16 bytes at a
 // time, gives the same numbers at a quarter of the operand rate: 140 cycles
 // per MMA.
@@ -403,9 +403,13 @@ __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_c
     if (warp == 0) tc::tmem_dealloc(tmem, a.p.columns);
 }
 
-// The rows and planes of a CTA that take the least time on 148 SMs, in cycles:
-// the MMAs (45 each, measured from the issuing warp), the box through L2, the
-// epilogue, and what a wave costs anyway.
+// The rows and planes of a CTA that take the least time on 148 SMs, from a fit
+// to 174 strips of 16 -> 16 at 64^3, 8 x 64^3, 128^3 and 128 x 128 x 64: a wave
+// of r CTAs per SM (by shared memory and TMEM) costs 10 us for the box, the
+// launch and the epilogue, and per MMA of a CTA 20 ns and 11 ns more for each of
+// the r that share the tensor pipe.  Its picks take 23.0, 152.7, 158.1 and
+// 89.6 us; the best strips 23.0, 143.0, 158.1 and 89.6.  (Counting the parts of
+// one CTA in cycles picked 26.9, 158.5, 158.2 and 98.6.)
 template <int CIN, int COUT>
 bool slab_plan(const VolumeShape& s, SlabPlan& best) {
     using L = SlabSmem<CIN, COUT>;
@@ -424,10 +428,11 @@ bool slab_plan(const VolumeShape& s, SlabPlan& best) {
             if (p.columns > 512u || smem > kSlabMaxSmem) break;
             p.smem = static_cast<uint32_t>(smem);
             const uint64_t ctas = static_cast<uint64_t>(s.batch) * ((s.z + bz - 1) / bz) * ((s.y + by - 1) / by);
-            const double waves = static_cast<double>((ctas + 147) / 148);
-            const double cycles = 27.0 * (bz * p.tiles * (CIN / 16) * 45.0 + 60.0) + smem / 40.0 + bz * p.tiles * 12.0 * COUT + 5000.0;
-            if (least == 0.0 || waves * cycles < least) {
-                least = waves * cycles;
+            const uint64_t resident = std::min({227ull * 1024u / (smem + 1024u), 512ull / p.columns, (ctas + 147ull) / 148u});
+            const double waves = static_cast<double>((ctas + 148u * resident - 1u) / (148u * resident));
+            const double cost = 10.0 + 27.0 * (bz * p.tiles * (CIN / 16)) * (0.020 + 0.011 * static_cast<double>(resident));
+            if (least == 0.0 || waves * cost < least) {
+                least = waves * cost;
                 best = p;
             }
         }
@@ -455,8 +460,8 @@ XsStatus launch_conv_forward(cudaStream_t st, const VolumeShape& s, const __nv_b
     uint32_t bx, by, bz;
     if (!conv_tile(s, bx, by, bz)) return XS_INVALID_ARGUMENT;
     // The slab wins where the 27 shifted boxes of narrow layers fill the SMs:
-    // 16 -> 16 at 64^3 26 us against 46 from the boxes, at 8 x 64^3 159
-    // against 294; 16 -> 32 at 8 x 32^3 38 against 48.  With fewer voxels a CTA
+    // 16 -> 16 at 64^3 23 us against 46 from the boxes, at 8 x 64^3 153
+    // against 294; 16 -> 32 at 8 x 32^3 29 against 48.  With fewer voxels a CTA
     // has too few MMAs behind one box to wait for (16 -> 32 at 32^3 14.1 us
     // against 11.1; by both slopes they meet near 100,000 voxels), and from 32
     // channels on a box fills an MMA's time anyway (32 -> 16 at 8 x 32^3 52.0
