@@ -97,6 +97,9 @@ def test_pcg_step_matches_reference_kernels_with_converged_sweeps(cuda):
     1e-6 themselves would not do: Gauss-Seidel's error at a given residual is
     dominated by smooth modes and measured 2.8e-5 on v at 24^3."""
     from common import product_domain, reference_step
+    from oracle import ref_binding as rb
+    if not rb.available():
+        pytest.skip("reference harness not built")
     cfg = with_solver(scenario("plume", res=(24, 24, 24)), "pcg", iterations=20000, tolerance=1e-6)
     res = tuple(cfg.resolution)
     st, ctl = seeded_state(res, seed=25, amp=0.2), seeded_control(res, seed=26)

@@ -9,7 +9,8 @@
   red-black Gauss-Seidel iterated until the FP32 sweeps stop lowering the
   residual: about 3e-6 relative at 64^3, 1e-5 at 128^3).  Density, temperature and
   velocity must agree to 1e-5 relative L2.
-  Run with the plain zero start, the classical warm start (ring of previous
+  Where the reference harness is not built (oracle/_ref), against the oracle
+  alone.  Run with the plain zero start, the classical warm start (ring of previous
   solutions, coarse-grid step) and the benchmark's learned pipeline.
 * The 256^3 headline pipeline (float4 fast paths, three-level coarse start,
   network step, smoothed PCG): one step after a 30-step rollout against the
@@ -26,6 +27,7 @@ from common import (PLUME_PARAMS, ROOT, field_errors, from_model_state, product_
                     seeded_control, to_model_state)
 
 from oracle import binding as ob
+from oracle import ref_binding as rb
 
 pytestmark = pytest.mark.gpu
 
@@ -84,7 +86,7 @@ def test_plume_rollout_matches_oracle_and_reference_kernels(cuda, n, start, step
     zero_control = ob.zeros_control(tuple(cfg.resolution), np.float64)
     ob.set_threads(os.cpu_count() or 1)
     P = ob.Problem(plume(n), "f64", solver="pcg", iterations=50000, tolerance=1e-12)
-    worst = {"oracle": 0.0, "reference": 0.0}
+    worst = {}
     for step in range(steps):
         check = step % every == every - 1
         if check:
@@ -97,20 +99,22 @@ def test_plume_rollout_matches_oracle_and_reference_kernels(cuda, n, start, step
             got = from_model_state(model, nxt)
             want, _, ost, _ = P.forward_step(before, zero_control, PLUME_PARAMS, guess=ctx.pressure_fields()[0].double().cpu().numpy())
             assert ost.converged == 1
-            ref, sweeps, residual = reference_step(plume(n), product_domain(ctx), before, zero_control, PLUME_PARAMS, tolerance=1e-9)
-            e_oracle, e_ref = field_errors(got, want), field_errors(got, ref)
-            report(f"rollout{n}_{start}", step=step + 1, oracle=e_oracle, reference=e_ref, reference_sweeps=sweeps,
-                   reference_residual=residual, product_iterations=stats["iterations"], product_residual=stats["final_residual"],
-                   warm_start_used=stats["warm_start_used"])
-            # the reference's FP32 sweeps stop at their rounding floor (the
-            # stall test of the harness: ~3e-6 relative at 64^3, ~1e-5 at
-            # 128^3); that they got there and not stuck early is checked here,
-            # the fields below
-            assert residual < 3e-5, (step, sweeps, residual)
-            for name, e in (("oracle", e_oracle), ("reference", e_ref)):
+            errors = {"oracle": field_errors(got, want)}
+            if rb.available():
+                ref, sweeps, residual = reference_step(plume(n), product_domain(ctx), before, zero_control, PLUME_PARAMS, tolerance=1e-9)
+                errors["reference"] = field_errors(got, ref)
+                # the reference's FP32 sweeps stop at their rounding floor (the
+                # stall test of the harness: ~3e-6 relative at 64^3, ~1e-5 at
+                # 128^3); that they got there and not stuck early is checked
+                # here, the fields below
+                assert residual < 3e-5, (step, sweeps, residual)
+                report(f"rollout{n}_{start}_reference", step=step + 1, sweeps=sweeps, residual=residual)
+            report(f"rollout{n}_{start}", step=step + 1, **errors, product_iterations=stats["iterations"],
+                   product_residual=stats["final_residual"], warm_start_used=stats["warm_start_used"])
+            for name, e in errors.items():
                 for field, v in e.items():
                     assert v < 1e-5, (start, step + 1, name, field, v)
-                worst[name] = max(worst[name], *e.values())
+                worst[name] = max(worst.get(name, 0.0), *e.values())
         cur, nxt = nxt, cur
     if network is not None:
         network.check()
