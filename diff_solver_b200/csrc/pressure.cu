@@ -1875,6 +1875,30 @@ __global__ void apply_operator_kernel(Operator op, const float* __restrict__ u, 
 __global__ void history_advance_kernel(uint32_t history, uint32_t* meta) {
     meta[1] = (min(meta[1], history - 1) + 1) % history;
     meta[0] = min(meta[0] + 1, history);
+    meta[kMetaPending] = 0u;
+}
+
+// history_keep: pressure into its slot, and by the last block to finish the
+// ring's new state.  A copy, bound by memory: a step takes 27 us more with it at
+// 256^3, 10 at 128^3 (combining the start in every step would take 175 at 256^3).
+__global__ void __launch_bounds__(256) history_keep_kernel(uint64_t n, const float* __restrict__ pressure, HistorySlots slots, uint32_t history,
+                                                           uint32_t* meta) {
+    const bool pending = meta[kMetaPending] != 0u;
+    const uint32_t valid = pending ? meta[kMetaKept] : meta[0], next = pending ? meta[kMetaKept + 1] : meta[1];
+    const uint32_t k = min(next, history - 1);
+    if (pending) {
+        float* dst = slots.s[k];
+        const uint64_t groups = n / 4, start = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+        for (uint64_t t = start; t < groups; t += static_cast<uint64_t>(gridDim.x) * blockDim.x) st4(dst + 4 * t, ld4(pressure + 4 * t));
+        if (start < n % 4) dst[4 * groups + start] = pressure[4 * groups + start];
+    }
+    __syncthreads();  // (the block has read meta)
+    if (threadIdx.x != 0 || atomicAdd(meta + kMetaTicket, 1u) != gridDim.x - 1u) return;
+    meta[kMetaTicket] = 0u;
+    meta[kMetaKept] = pending ? min(valid + 1u, history) : min(valid, history);
+    meta[kMetaKept + 1] = pending ? (k + 1u) % history : k;
+    meta[0] = meta[1] = 0u;
+    meta[kMetaPending] = 1u;
 }
 
 bool coarse_grid(const Grid& g, uint32_t coarsening, Grid& coarse) {
@@ -2246,7 +2270,9 @@ __global__ void jacobi_sweep_kernel(Operator op, const T* __restrict__ rhs, cons
 
 XsStatus jacobi_sweeps(cudaStream_t st, const Grid& g, uint32_t anchor, const uint32_t* mask, const XsScalarBoundary& pb, const float* rhs,
                        const double* rhs_d, const float* x, float* tmp, float* x_out, int sweeps) {
-    if (!x || !tmp || !x_out || x_out == x || x_out == tmp || (!rhs && !rhs_d) || sweeps < 0) return XS_INVALID_ARGUMENT;
+    // in place where the first sweep goes to tmp
+    const bool in_place = x_out == x && (sweeps == 0 || sweeps % 2 != 0);
+    if (!x || !tmp || !x_out || in_place || x_out == tmp || (!rhs && !rhs_d) || sweeps < 0) return XS_INVALID_ARGUMENT;
     const Operator op{g, mask, anchor, pb, rhs_d == nullptr};
     const uint64_t n = cell_count(g);
     const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 148 * 16));
@@ -2366,11 +2392,11 @@ XsStatus coarse_cycles(cudaStream_t st, const Grid& g, uint32_t anchor, const Xs
     if (cycles < 1 || !out) return XS_INVALID_ARGUMENT;
     const float* x = h.ring_start;
     for (int c = 0; c < cycles; ++c) {
-        float* dst = (c % 2 == 0) ? h.start : h.ring_start;  // never x
+        // (an even number of sweeps works in place and leaves the ring's start as it is)
+        const int sweeps = rhs_d ? kAdjointPreSweeps : kCoarsePreSweeps;
+        float* dst = (c % 2 == 0 || sweeps % 2 == 0) ? h.start : h.ring_start;
         XsStatus s;
-        if ((s = jacobi_sweeps(st, g, anchor, nullptr, pb, rhs, rhs_d, x, h.extra_product, dst, rhs_d ? kAdjointPreSweeps : kCoarsePreSweeps)) !=
-            XS_OK)
-            return s;
+        if ((s = jacobi_sweeps(st, g, anchor, nullptr, pb, rhs, rhs_d, x, h.extra_product, dst, sweeps)) != XS_OK) return s;
         if ((s = start_residual(st, g, anchor, nullptr, pb, rhs, dst, h.residual, rhs_d)) != XS_OK) return s;
         if ((s = coarse_correction(st, g, anchor, pb, h, h.residual, c == 0 ? kCoarseMaxIterations : kLaterCoarseIterations)) != XS_OK) return s;
         if ((s = line_step(st, g, anchor, nullptr, pb, h, h.correction, dst, h.residual, dst, keep_residual && c == cycles - 1)) != XS_OK)
@@ -2458,9 +2484,32 @@ XsStatus history_push(cudaStream_t st, const Grid& g, uint32_t anchor, const uin
     return check_launch();
 }
 
+XsStatus history_keep(cudaStream_t st, const Grid& g, const WarmHistory& h, const float* pressure) {
+    if (h.history == 0) return XS_OK;
+    HistorySlots slots{};
+    for (uint32_t i = 0; i < h.history; ++i) slots.s[i] = h.slots[i];
+    const uint64_t n = cell_count(g);
+    history_keep_kernel<<<static_cast<unsigned>(std::min<uint64_t>((n / 4 + 255) / 256 + 1, 148 * 8)), 256, 0, st>>>(n, pressure, slots, h.history, h.meta);
+    return check_launch();
+}
+
+XsStatus kept_start(cudaStream_t st, const Grid& g, uint32_t anchor, const uint32_t* mask, const XsScalarBoundary& pb, const WarmHistory& h,
+                    const float* rhs, float* out) {
+    const Operator op{g, mask, anchor, pb, true};
+    const unsigned blocks = static_cast<unsigned>(std::min<uint64_t>((cell_count(g) + 255) / 256, 148 * 16));
+    for (uint32_t i = 0; i < h.history; ++i) {
+        apply_operator_kernel<<<blocks, 256, 0, st>>>(op, h.slots[i], h.products[i]);
+        const XsStatus s = check_launch();
+        if (s != XS_OK) return s;
+    }
+    WarmHistory kept = h;
+    kept.meta += kMetaKept;
+    return galerkin_combine(st, g, anchor, mask, pb, kept, true, nullptr, 0, rhs, out);
+}
+
 XsStatus history_reset(cudaStream_t st, const WarmHistory& h) {
     if (h.history == 0 || !h.meta) return XS_OK;
-    return check_cuda(cudaMemsetAsync(h.meta, 0, 2 * sizeof(uint32_t), st));
+    return check_cuda(cudaMemsetAsync(h.meta, 0, kMetaKept * sizeof(uint32_t), st));
 }
 
 XsStatus read_solve_stats(cudaStream_t stream, const void* workspace, const Grid& g, XsSolveStats* out) {

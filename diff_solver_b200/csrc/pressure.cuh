@@ -86,12 +86,18 @@ XsStatus read_solve_stats(cudaStream_t stream, const void* workspace, const Grid
 // at most one extra vector (kMaxBasis in all) spanning the Galerkin start.
 constexpr int kMaxHistory = 5;
 constexpr int kMaxBasis = kMaxHistory + 1;
+// State of the ring on the device (WarmHistory::meta): [0] valid slots, [1] next
+// slot, whose products are stored too (history_push).  For solves that do not
+// start from the ring (history_keep): whether the last solution has still to
+// enter it, a ticket of the kernel that enters it, and, from kMetaKept on,
+// valid slots and next slot as the last such solve found them.
+constexpr int kMetaPending = 2, kMetaTicket = 3, kMetaKept = 4;
 struct WarmHistory {
     float* slots[kMaxBasis];
     float* products[kMaxBasis];  // A slot, computed when the slot is written
     uint32_t history;   // ring slots (0: off)
     uint32_t forward_rounds;  // start rounds before a forward solve (0: defaults)
-    uint32_t* meta;     // device: [0] valid slots, [1] next slot
+    uint32_t* meta;     // device: see above
     float* start;       // the start vector of the last forward solve (N)
     float* ring_start;  // the Galerkin start from the ring alone (N)
     float* residual;    // b - A ring_start (N)
@@ -245,6 +251,15 @@ XsStatus start_residual(cudaStream_t st, const Grid& g, uint32_t anchor, const u
 // with its product by the operator.
 XsStatus history_push(cudaStream_t st, const Grid& g, uint32_t anchor, const uint32_t* mask, const XsScalarBoundary& pb, const WarmHistory& h,
                       const float* pressure, const double* pressure64 = nullptr);
+// Before a forward solve that does not start from the ring: the solution of
+// the solve before, still in `pressure`, enters the ring without its product,
+// unless a reset or a history_push came between.  The ring then stays as this
+// solve finds it until the next one, and kept_start gives the start that it
+// would have given (products formed anew).  A later solve that does start from
+// the ring finds it empty.
+XsStatus history_keep(cudaStream_t st, const Grid& g, const WarmHistory& h, const float* pressure);
+XsStatus kept_start(cudaStream_t st, const Grid& g, uint32_t anchor, const uint32_t* mask, const XsScalarBoundary& pb, const WarmHistory& h,
+                    const float* rhs, float* out);
 // Empties the ring.
 XsStatus history_reset(cudaStream_t st, const WarmHistory& h);
 

@@ -11,6 +11,14 @@
 
 namespace xs {
 
+// Whether a forward solve starts from the direct solve of its own grid: the
+// grid's operator separates, and the caller has not set the number of rounds.
+static bool starts_directly(const Grid& g, const XsPressureSolve& solve, uint32_t anchor, const uint32_t* mask, const XsScalarBoundary& pb,
+                            const WarmHistory* h, DirectPlan& plan) {
+    return solve.kind == XS_SOLVER_JACOBI_PCG && h && h->history > 0 && h->coarsening != 0 && mask == nullptr && h->direct && h->forward_rounds == 0 &&
+           direct_plan(g, mask, anchor, pb, true, plan);
+}
+
 // ------------------------------------------------------------ projection
 // operators.cu:1004-1013: rhs, pressure solve, gradient subtraction.  With
 // the PCG kind the velocity is corrected from the FP64 iterate.
@@ -42,13 +50,15 @@ XsStatus projection_forward(cudaStream_t st, const Grid& g, const XsPressureSolv
     float *guess = nullptr, *low = nullptr;
     const bool coarse = ring && history->coarsening != 0 && mask == nullptr;
     DirectPlan plan;
-    const bool direct = coarse && history->direct && history->forward_rounds == 0 && direct_plan(g, mask, anchor, pb, true, plan);
+    const bool direct = starts_directly(g, solve, anchor, mask, pb, history, plan);
     if (direct) {
         // the grid's operator separates: solved as it is, instead of the ring
-        // and the rounds (unless the caller set their number); the network's
-        // step then works on the residual this leaves
+        // and the rounds; the network's step then works on the residual this
+        // leaves.  The solutions are kept all the same, for the ring's start is
+        // what the network learns to correct (xs_smoke_warm_start_fields)
         const WarmHistory& h = *history;
         const float* x = nullptr;
+        if ((s = history_keep(st, g, h, pressure)) != XS_OK) return s;
         if ((s = direct_start<float>(st, g, pb, h, plan, rhs, &x, &low)) != XS_OK) return s;
         if (warm_start) {
             // the residual of both parts is the first part's less A low
@@ -79,10 +89,9 @@ XsStatus projection_forward(cudaStream_t st, const Grid& g, const XsPressureSolv
                 return s;
             }
             if (warm_start) {
-                float* out = x == h.start ? h.ring_start : h.start;
                 if ((s = warm_start_guess(warm_start, st, g, h.residual, &guess)) != XS_OK) return s;
-                if ((s = line_step(st, g, anchor, mask, pb, h, guess, x, h.residual, out, false)) != XS_OK) return s;
-                x = out;
+                if ((s = line_step(st, g, anchor, mask, pb, h, guess, x, h.residual, h.start, false)) != XS_OK) return s;
+                x = h.start;
             }
             used.initial_guess = x;
         }
@@ -485,8 +494,17 @@ XsStatus xs_smoke_warm_start_fields(cudaStream_t stream, const XsSmokeModel* mod
     if (!valid_model(model) || !workspace || model->warm_start_history == 0) return XS_INVALID_ARGUMENT;
     const Grid g = make_grid(model->grid);
     const StepWorkspace w = carve_step(workspace, g, XS_MODE_FORWARD, model->warm_start_history, model->warm_start_coarsening);
-    const XsStatus s = start_residual(stream, g, model->pressure_anchor, model->cell_mask, model->pressure_boundary, w.rhs, w.history.ring_start,
-                                      w.history.residual);
+    WarmHistory h = w.history;
+    h.forward_rounds = model->warm_start_rounds;
+    DirectPlan plan;
+    XsStatus s = XS_OK;
+    if (starts_directly(g, model->pressure, model->pressure_anchor, model->cell_mask, model->pressure_boundary, &h, plan)) {
+        // the step did not need it: combined here
+        s = kept_start(stream, g, model->pressure_anchor, model->cell_mask, model->pressure_boundary, h, w.rhs, h.ring_start);
+        if (s != XS_OK) return s;
+    }
+    s = start_residual(stream, g, model->pressure_anchor, model->cell_mask, model->pressure_boundary, w.rhs, w.history.ring_start,
+                       w.history.residual);
     if (s != XS_OK) return s;
     if (ring_start) *ring_start = w.history.ring_start;
     if (residual) *residual = w.history.residual;

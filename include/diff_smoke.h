@@ -344,8 +344,9 @@ typedef struct XsSmokeModel {
      * boundary value other than 0, at most 512 cells per axis, equal ends or
      * periodic x and y or z, the third axis not periodic) and
      * warm_start_rounds is 0, the system is solved there directly instead, in
-     * FP32, and neither ring nor rounds are used; the learned correction then
-     * works on the residual that leaves. */
+     * FP32, and neither ring nor rounds enter the start (the ring is kept for
+     * xs_smoke_warm_start_fields); the learned correction then works on the
+     * residual that leaves. */
     uint32_t warm_start_coarsening;
     /* rounds of sweeps and coarse-grid correction before a forward solve
      * (0: the defaults, two without a learned warm start and one before its
@@ -358,7 +359,9 @@ typedef struct XsSmokeModel {
      * [0] start, [1] sources and forces done, [2] integration, [3] advection
      * and constraint, [4] pressure right-hand side, [5] warm start (the fine
      * PCG launch follows), [6] fine pressure solve, [7] ring update,
-     * [8] projection, [9] scalar advection (end of the step). */
+     * [8] projection, [9] scalar advection (end of the step).  Before a
+     * direct solve the ring takes the solution of the step before, within
+     * [5]; [7] is then empty. */
     cudaEvent_t* stage_events;
 } XsSmokeModel;
 #define XS_STEP_STAGES 9
@@ -431,7 +434,8 @@ XsStatus xs_smoke_pressure_fields(const XsSmokeModel* model, void* workspace, fl
 
 /* With a ring of previous solutions: device pointers, inside the workspace,
  * of the ring's Galerkin start x0 of the last forward solve and of its
- * residual b - A x0 (recomputed on the stream by this call): with the
+ * residual b - A x0 (recomputed on the stream by this call, x0 as well where
+ * the solve started directly; model as it was for that step): with the
  * solution, the (residual, correction) pairs the network learns when it
  * serves a model that keeps a ring. */
 XsStatus xs_smoke_warm_start_fields(cudaStream_t stream, const XsSmokeModel* model, void* workspace, float** ring_start, float** residual);
