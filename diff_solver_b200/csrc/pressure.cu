@@ -37,7 +37,20 @@ namespace xs {
 // ------------------------------------------------------------------ layout
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
-PressureWorkspace carve_pressure_workspace(void* base, const Grid& g) {
+// Whether a grid gets padded vectors: where a form that works on them may
+// serve it.  Those that keep the grid in the SMs hold up to kResidentCells; the
+// marching one serves grids with a mask or rows that are no multiple of 4
+// (launch_cg_any), rows of up to kMarchPitch.  They cost 9 to 10 bytes a cell
+// (45.6 against 36.0 at 512^3), so past kPaddedCells, where a differentiable
+// step takes about 100 of a device's 180 GB, grids keep the general kernels
+// and with them the memory they always took.
+static bool wants_padding(const Grid& g, uint64_t padded, bool masked) {
+    const uint64_t n = cell_count(g);
+    if (n > kPaddedCells || padded > padded_limit(n) || padded >= (1ull << 31)) return false;
+    return n <= kResidentCells || (static_cast<uint32_t>(g.nx) < kMarchPitch && (masked || g.nx % 4 != 0));
+}
+
+PressureWorkspace carve_pressure_workspace(void* base, const Grid& g, bool masked) {
     const size_t n = cell_count(g);
     PressureWorkspace w{};
     char* p = static_cast<char*>(base);
@@ -53,7 +66,7 @@ PressureWorkspace carve_pressure_workspace(void* base, const Grid& g) {
     w.x64 = static_cast<double*>(take(sizeof(double) * n));
     // sized for periodic axes, which pad most: the boundary modes come with the solve
     const uint64_t padded = padded_cells(g, {2u, 2u, 2u, 2u, 2u, 2u});
-    const bool pad = padded <= padded_limit(n) && padded < (1ull << 31);
+    const bool pad = wants_padding(g, padded, masked);
     const size_t bytes = sizeof(float) * (pad ? padded : n);
     w.z = static_cast<float*>(take(bytes));
     w.p0 = static_cast<float*>(take(bytes));
@@ -92,7 +105,7 @@ PadExtents pad_extents(const Grid& g, const uint32_t (&modes)[6]) {
 
 uint64_t padded_cells(const Grid& g, const uint32_t (&modes)[6]) { return pad_extents(g, modes).total; }
 
-size_t pressure_workspace_bytes(const Grid& g) { return carve_pressure_workspace(nullptr, g).bytes; }
+size_t pressure_workspace_bytes(const Grid& g, bool masked) { return carve_pressure_workspace(nullptr, g, masked).bytes; }
 
 // ------------------------------------------------------------ the operator
 struct Operator {
@@ -1336,8 +1349,9 @@ bool launch_cg_resident(CgArgs& a, uint32_t resident, cudaStream_t stream, XsSta
 //    16.2, 128^3 26 -> 21.  From 144^3 on, and for warm starts of a dozen
 //    iterations (128^3: 0.42 against 0.48 ms), the two-pass kernel's lighter
 //    set-up and larger occupancy win: 160^3 36 against 38, 256^3 120 against 141;
-//  * false: neither (rows of more than 764 cells leave the marching form's
-//    runs too short, thin grids the padding too large).
+//  * false: neither (rows of more than 767 cells leave the marching form's
+//    runs too short, thin grids the padding too large; grids past kPaddedCells
+//    have no padded vectors).
 template <bool kSmooth>
 bool launch_cg_any(CgArgs& a, int sms, cudaStream_t stream, XsStatus& status) {
     const uint32_t resident = std::min<uint32_t>(kMaxCgBlocks, static_cast<uint32_t>(sms));
@@ -1347,7 +1361,8 @@ bool launch_cg_any(CgArgs& a, int sms, cudaStream_t stream, XsStatus& status) {
     if (a.c.use_fast && (kSmooth || a.g.n > 2500000u)) return false;
     constexpr uint32_t span = kMarchPer * kCgThreads;
     const uint32_t halo = a.g.pitch / 4, plane_quads = halo * a.g.ny;
-    if (8 * halo > 3 * span) return false;
+    static_assert(8 * (kMarchPitch / 4) <= 3 * span);
+    if (a.g.pitch > kMarchPitch) return false;
     const uint32_t most = span - 2 * halo;
     // equal runs; the slabs that leave the least work to the busiest block (a
     // slab's ends cost about a plane and a half)
@@ -1437,7 +1452,7 @@ XsStatus solve_pressure(cudaStream_t stream, const Grid& g, const XsPressureSolv
                         const XsScalarBoundary& pb, const float* rhs_f, const double* rhs_d, float* pressure_out,
                         double* solution_out, void* workspace, PressureWorkspace* carved, const float* guess_low) {
     if (!workspace) return XS_INVALID_ARGUMENT;
-    const PressureWorkspace w = carve_pressure_workspace(workspace, g);
+    const PressureWorkspace w = carve_pressure_workspace(workspace, g, mask != nullptr);
     if (carved) *carved = w;
     DeviceLimits lim;
     XsStatus s = device_limits(lim);
@@ -1880,7 +1895,7 @@ __global__ void history_advance_kernel(uint32_t history, uint32_t* meta) {
 
 // history_keep: pressure into its slot, and by the last block to finish the
 // ring's new state.  A copy, bound by memory: a step takes 27 us more with it at
-// 256^3, 10 at 128^3 (combining the start in every step would take 175 at 256^3).
+// 256^3, 10 at 128^3 (combining the start in every step: about 200 at 256^3).
 __global__ void __launch_bounds__(256) history_keep_kernel(uint64_t n, const float* __restrict__ pressure, HistorySlots slots, uint32_t history,
                                                            uint32_t* meta) {
     const bool pending = meta[kMetaPending] != 0u;
@@ -1931,13 +1946,13 @@ size_t warm_history_bytes(const Grid& g, uint32_t history, uint32_t coarsening) 
     Grid c, c2;
     if (coarse_grid(g, coarsening, c)) {
         const size_t nc = cell_count(c);
-        bytes += align_up(n * 4, 256) + align_up(nc * 8, 256) + align_up(nc * 4, 256) + align_up(pressure_workspace_bytes(c), 256);
+        bytes += align_up(n * 4, 256) + align_up(nc * 8, 256) + align_up(nc * 4, 256) + align_up(pressure_workspace_bytes(c, false), 256);
         if (direct_fits(g)) bytes += align_up(direct_basis_bytes(), 256);
         if (spectral_fits(c)) bytes += align_up(4 * 6 * kSpectralMax * kSpectralMax, 256) + align_up(4 * 3 * kSpectralMax, 256);
         const uint32_t f2 = second_coarsening(c);
         if (f2 && coarse_grid(c, f2, c2)) {
             const size_t nc2 = cell_count(c2);
-            bytes += 5 * align_up(nc * 4, 256) + align_up(nc2 * 8, 256) + align_up(nc2 * 4, 256) + align_up(pressure_workspace_bytes(c2), 256);
+            bytes += 5 * align_up(nc * 4, 256) + align_up(nc2 * 8, 256) + align_up(nc2 * 4, 256) + align_up(pressure_workspace_bytes(c2, false), 256);
         }
     }
     return bytes;
@@ -1972,7 +1987,7 @@ WarmHistory carve_warm_history(void* base, const Grid& g, uint32_t history, uint
         h.correction = reinterpret_cast<float*>(take(n * 4));
         h.coarse_rhs = reinterpret_cast<double*>(take(nc * 8));
         h.coarse_solution = reinterpret_cast<float*>(take(nc * 4));
-        h.coarse_solver = take(pressure_workspace_bytes(h.coarse));
+        h.coarse_solver = take(pressure_workspace_bytes(h.coarse, false));
         if (direct_fits(g)) h.direct = take(direct_basis_bytes());
         if (spectral_fits(h.coarse)) {
             h.spectral_basis = reinterpret_cast<float*>(take(4 * 6 * kSpectralMax * kSpectralMax));
@@ -1989,7 +2004,7 @@ WarmHistory carve_warm_history(void* base, const Grid& g, uint32_t history, uint
             h.coarse_correction = reinterpret_cast<float*>(take(nc * 4));
             h.coarsest_rhs = reinterpret_cast<double*>(take(nc2 * 8));
             h.coarsest_solution = reinterpret_cast<float*>(take(nc2 * 4));
-            h.coarsest_solver = take(pressure_workspace_bytes(h.coarsest));
+            h.coarsest_solver = take(pressure_workspace_bytes(h.coarsest, false));
         }
     }
     return h;

@@ -46,6 +46,9 @@ constexpr uint64_t padded_limit(uint64_t cells) { return cells + cells / 4 + 163
 // sums of 16 bytes each.
 constexpr int kMaxCgBlocks = 160;
 constexpr size_t kSlotBytes = 2ull * kMaxCgBlocks * 16 * 16;
+constexpr uint64_t kResidentCells = 512ull * 8 * 8 * kMaxCgBlocks;  // most cells of the forms that keep the grid in the SMs
+constexpr uint64_t kPaddedCells = 1ull << 27;
+constexpr uint32_t kMarchPitch = 768;  // longest padded row of the marching form
 
 // Division by a runtime constant for numerators below 2^31:
 // q = (n * m) >> shift with m = floor(2^shift / d) + 1, shift = 31 + ceil(log2 d).
@@ -64,8 +67,10 @@ struct FastGeom {
     uint32_t kind[6];
 };
 
-PressureWorkspace carve_pressure_workspace(void* base, const Grid& g);
-size_t pressure_workspace_bytes(const Grid& g);
+// masked: for solves with a cell mask too.  The layout up to x64 is the same
+// with and without one, and the one with it is never the smaller.
+PressureWorkspace carve_pressure_workspace(void* base, const Grid& g, bool masked = true);
+size_t pressure_workspace_bytes(const Grid& g, bool masked = true);
 
 // Solves the pressure system for rhs_f (forward, FP32, fixed boundary values
 // enter b) or rhs_d (adjoint, FP64, no fixed values).  pressure_out receives

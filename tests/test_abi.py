@@ -101,6 +101,30 @@ def test_largest_grids_within_32_bit_indexing_are_accepted():
     assert lib.xs_projection_workspace_bytes(_native.XsGrid(512, 512, 256, 1 / 512, 1 / 1024)) > 0
 
 
+def test_workspaces_hold_no_vectors_that_no_solve_uses():
+    """The pressure solver's vectors: FP64 iterate and seven FP32 vectors, 36
+    bytes a cell.  The padded forms' extra ones (9 to 10 bytes) are there for
+    the grids they serve, not past 2^27 cells (where the largest grids of a
+    device are), for rows longer than they take, nor for coarse grids of
+    aligned rows past the ones kept in the SMs."""
+    lib = _native.lib()
+
+    def solver(*extents):
+        return (lib.xs_projection_workspace_bytes(_native.XsGrid(*extents, 1e-3, 5e-4)) - (1 << 20)) / (extents[0] * extents[1] * extents[2])
+
+    for extents in ((640, 640, 512), (515, 515, 515), (800, 800, 800), (1000, 100, 100)):
+        assert solver(*extents) <= 36.0, (extents, solver(*extents))
+    for extents in ((200, 190, 180), (767, 100, 100), (130, 130, 130), (512, 512, 512)):
+        assert 45.0 < solver(*extents) < 50.0, (extents, solver(*extents))
+    m = _native.XsSmokeModel()
+    m.grid = _native.XsGrid(512, 512, 256, 1 / 512, 1 / 1024)
+    base = lib.xs_smoke_workspace_bytes(ctypes.byref(m), 0)
+    m.warm_start_history, m.warm_start_coarsening = 5, 2
+    # 5 solutions, their products, 5 vectors; an eighth of 12 + 36 bytes and of
+    # 20 bytes on the coarse grid; the coarsest grid's share is below 0.2
+    assert lib.xs_smoke_workspace_bytes(ctypes.byref(m), 0) - base <= (4 * 15 + (12 + 36 + 20) / 8 + 0.2) * 512 * 512 * 256
+
+
 def test_warm_start_options_are_validated_without_gpu():
     """The ring (0..5 solutions) and the coarse-grid correction (a factor that
     divides the grid, with a ring and no colliders) size the workspace; other
