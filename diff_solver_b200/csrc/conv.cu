@@ -525,17 +525,77 @@ struct WgradLayout {
     static constexpr uint32_t total = 1024u + stages * stage_bytes + 256u;
 };
 
+constexpr uint32_t kWgradCtas = 148u;  // most CTAs of a weight gradient, one per SM
+
 struct WgradArgs {
     VolumeShape s;
     uint32_t bx, by, bz;
     uint32_t tiles;
     float* partial;  // [gridDim.x][27][COUT][CIN]
     int* error;
+    // After slabs: their CTAs' flags and a ticket.  Without a flag set their sums
+    // are added up here; with one the sums are formed again, and added up by
+    // the last CTA to finish.
+    const uint32_t* redo;  // null: not after slabs
+    uint32_t redo_count;
+    uint32_t* ticket;
+    float* dw;
+    int accumulate;
+};
+
+// dW[i] (+)= sum over CTAs of partial[cta][i], in CTA order, for i = first,
+// first + step, ... (kSums of them), with 32 loads of each in flight.
+template <int kSums>
+struct PartialSums {
+    float acc[kSums];
+    __device__ __forceinline__ void form(const float* partial, uint32_t ctas, uint32_t count, uint32_t first, uint32_t step) {
+#pragma unroll
+        for (int k = 0; k < kSums; ++k) acc[k] = 0.0f;
+        for (uint32_t c0 = 0; c0 < ctas; c0 += 32u) {
+            float v[kSums][32];
+#pragma unroll
+            for (int k = 0; k < kSums; ++k)
+#pragma unroll
+                for (uint32_t c = 0; c < 32u; ++c)
+                    if (c0 + c < ctas && first + k * step < count) v[k][c] = __ldcg(partial + static_cast<size_t>(c0 + c) * count + first + k * step);
+#pragma unroll
+            for (int k = 0; k < kSums; ++k)
+#pragma unroll
+                for (uint32_t c = 0; c < 32u; ++c)
+                    if (c0 + c < ctas && first + k * step < count) acc[k] += v[k][c];
+        }
+    }
+    __device__ __forceinline__ void add_to(float* dw, int accumulate, uint32_t count, uint32_t first, uint32_t step) const {
+#pragma unroll
+        for (int k = 0; k < kSums; ++k) {
+            const uint32_t i = first + k * step;
+            if (i < count) dw[i] = accumulate ? dw[i] + acc[k] : acc[k];
+        }
+    }
 };
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_constant__ CUtensorMap x_map,
                                                                    const __grid_constant__ CUtensorMap dy_map, WgradArgs a) {
+    constexpr uint32_t count = 27u * CIN * COUT;
+    if (a.redo) {
+        // the sums are formed while the flags are on their way; a CTA per SM
+        // (more do not fit beside the boxes' memory)
+        constexpr int kSums = (count + kWgradCtas * kConvThreads - 1u) / (kWgradCtas * kConvThreads);
+        const uint32_t first = (blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x, step = gridDim.x * gridDim.y * blockDim.x;
+        bool any = false;
+        for (uint32_t i = threadIdx.x; i < a.redo_count; i += blockDim.x) any |= __ldcg(a.redo + i) != 0u;
+        PartialSums<kSums> sums;
+        sums.form(a.partial, a.redo_count, count, first, step);
+        if (!__syncthreads_or(any)) {
+            sums.add_to(a.dw, a.accumulate, count, first, step);
+            for (uint32_t i = first + kSums * step; i < count; i += kSums * step) {
+                sums.form(a.partial, a.redo_count, count, i, step);
+                sums.add_to(a.dw, a.accumulate, count, i, step);
+            }
+            return;
+        }
+    }
     using L = WgradLayout<CIN, COUT>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
@@ -646,6 +706,19 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_
     tc::tc_fence_before();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, 256);
+    if (!a.redo) return;
+    __shared__ uint32_t before;
+    __threadfence();  // the CTA's sums before its ticket
+    __syncthreads();
+    if (threadIdx.x == 0) before = atomicAdd(a.ticket, 1u);
+    __syncthreads();
+    if (before != gridDim.x * gridDim.y - 1u) return;
+    __threadfence();
+    PartialSums<1> sums;
+    for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) {
+        sums.form(a.partial, nctas, count, i, 0u);
+        sums.add_to(a.dw, a.accumulate, count, i, 0u);
+    }
 }
 
 // -------------------------------------------- weight gradient, read once
@@ -666,7 +739,9 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_
 // 8 x 64^3: 82.8 us (298), where the MMAs, 128 x 48 x 16 at 45 cycles, are 65.
 //
 // A voxel that is infinite or NaN also meets zeros here that no tap pairs it
-// with (a row's margin): more taps of the sums turn NaN than those it is in.
+// with (a row's margin), which turn taps NaN that it is not in.  A CTA whose
+// sums are not all finite raises its flag, and the kernel that would add up the
+// CTAs' sums then forms them again from boxes.
 constexpr uint64_t kWslabMinVoxels = 30000u;
 constexpr uint32_t kWsTail = 32u;  // voxels of zeros past a plane: a K step's rest and the atoms' shifts
 
@@ -677,6 +752,8 @@ struct WslabArgs {
     uint32_t slots;     // planes in flight
     uint32_t x_bytes, slot_bytes;
     float* partial;     // [gridDim.x][27][COUT][CIN]
+    uint32_t* redo;     // [gridDim.x]: 1 where a sum is not finite
+    uint32_t* ticket;   // of what follows, cleared here
     int* error;
 };
 constexpr uint32_t kWsMaxSlots = 8u;
@@ -784,6 +861,7 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_slab_kernel(const __
     __syncwarp();
     const bool got = tc::mbar_wait(accum, 0);
     tc::tc_fence_after();
+    bool finite = true;
     if (got && warp * 32 < 3 * CIN) {
         const int m = warp * 32 + lane, dx = m / CIN, ci = m % CIN;
         for (int d = 0; d < 9; ++d) {  // planes of dY in rising order fall to taps of falling dz, rows to dy
@@ -795,14 +873,21 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_slab_kernel(const __
                 if (dx < 3) {
                     float* dst = a.partial + ((static_cast<size_t>(blockIdx.x) * 27 + tap) * COUT + c0) * CIN + ci;
 #pragma unroll
-                    for (int q = 0; q < 16; ++q) dst[static_cast<size_t>(q) * CIN] = v[q];
+                    for (int q = 0; q < 16; ++q) {
+                        dst[static_cast<size_t>(q) * CIN] = v[q];
+                        finite &= isfinite(v[q]);
+                    }
                 }
             }
         }
     }
     if ((!ok || !got) && a.error) atomicExch(a.error, 1);
     tc::tc_fence_before();
-    __syncthreads();
+    const bool again = __syncthreads_or(!finite) != 0;
+    if (threadIdx.x == 0) {
+        a.redo[blockIdx.x] = again ? 1u : 0u;
+        if (blockIdx.x == 0) *a.ticket = 0u;
+    }
     if (warp == 0) tc::tmem_dealloc(tmem, columns);
 }
 
@@ -824,30 +909,32 @@ bool wgrad_slab_plan(const VolumeShape& s, uint32_t ctas, WslabArgs& best) {
         const uint64_t cycles = of_one * (3u * ((rows * px + 15u) / 16u) * 45u + 200u) + 2u * (of_one / s.z + 1u) * 400u;
         if (least == 0u || cycles < least) {
             least = cycles;
-            best = WslabArgs{s, rows, strips, slots, x_bytes, slot, nullptr, nullptr};
+            best = WslabArgs{s, rows, strips, slots, x_bytes, slot, nullptr, nullptr, nullptr, nullptr};
         }
     }
     return least > 0u;
 }
 
-// dW[i] (+)= sum over CTAs of partial[cta][i], in CTA order.
+// dW (+)= the sums over CTAs of their parts.
 __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, uint32_t ctas, uint32_t count, float* __restrict__ dw, int accumulate) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    float acc = 0.0f;
-    for (uint32_t c = 0; c < ctas; ++c) acc += partial[static_cast<size_t>(c) * count + i];
-    dw[i] = accumulate ? dw[i] + acc : acc;
+    PartialSums<1> sums;
+    sums.form(partial, ctas, count, i, 0u);
+    sums.add_to(dw, accumulate, count, i, 0u);
 }
 
 uint32_t wgrad_ctas(const VolumeShape& s) {
     uint32_t bx, by, bz;
     if (!conv_tile(s, bx, by, bz)) return 0;
     const uint64_t tiles = static_cast<uint64_t>(s.batch) * (s.z / bz) * (s.y / by) * (s.x / bx);
-    return static_cast<uint32_t>(tiles < 148 ? tiles : 148);
+    return static_cast<uint32_t>(tiles < kWgradCtas ? tiles : kWgradCtas);
 }
 
+// (the partial sums, and behind them a flag per CTA and a ticket)
 size_t wgrad_partial_floats(const VolumeShape& s, int cin, int cout) {
-    return static_cast<size_t>(wgrad_ctas(s)) * 27u * static_cast<size_t>(cin) * static_cast<size_t>(cout);
+    const size_t ctas = wgrad_ctas(s);
+    return ctas == 0 ? 0 : ctas * (27u * static_cast<size_t>(cin) * static_cast<size_t>(cout) + 1u) + 1u;
 }
 
 template <int CIN, int COUT>
@@ -864,6 +951,7 @@ XsStatus launch_wgrad(cudaStream_t st, const VolumeShape& s, const __nv_bfloat16
     const uint32_t tiles = static_cast<uint32_t>(static_cast<uint64_t>(s.batch) * (s.z / bz) * (s.y / by) * (s.x / bx));
     const uint32_t ctas = wgrad_ctas(s);
     const uint32_t count = 27u * CIN * COUT;
+    WgradArgs args{s, bx, by, bz, tiles, partial, error, nullptr, 0u, nullptr, dw, accumulate ? 1 : 0};
     if constexpr (CIN <= 32 && COUT <= 32) {
         // 16 -> 16 at 8 x 64^3 82.8 us against 298 from the boxes, at 64^3 22.9
         // against 48.0, at 32^3 14.5 against 16.5, where a CTA has 6 planes
@@ -871,7 +959,9 @@ XsStatus launch_wgrad(cudaStream_t st, const VolumeShape& s, const __nv_bfloat16
         // first three loads; 32 -> 32 at 8 x 32^3 20.3 against 55.
         WslabArgs slab{};
         if (static_cast<uint64_t>(s.x) * s.y * s.z * s.batch >= kWslabMinVoxels && wgrad_slab_plan<CIN, COUT>(s, ctas, slab)) {
-            if (!make_activation_map(&xm, x, s, CIN, s.x + 1u, slab.rows, 1) || !make_activation_map(&ym, dy, s, COUT, s.x + 1u, slab.rows + 2u, 1))
+            CUtensorMap xs_map, dys_map;
+            if (!make_activation_map(&xs_map, x, s, CIN, s.x + 1u, slab.rows, 1) ||
+                !make_activation_map(&dys_map, dy, s, COUT, s.x + 1u, slab.rows + 2u, 1))
                 return XS_CUDA_ERROR;
             static DeviceOnce slab_configured;
             if (!slab_configured.run([] {
@@ -879,15 +969,21 @@ XsStatus launch_wgrad(cudaStream_t st, const VolumeShape& s, const __nv_bfloat16
                 }))
                 return XS_CUDA_ERROR;
             slab.partial = partial;
+            slab.redo = reinterpret_cast<uint32_t*>(partial + static_cast<size_t>(ctas) * count);
+            slab.ticket = slab.redo + ctas;
             slab.error = error;
             const uint32_t planes = s.batch * slab.strips * s.z, slab_ctas = std::min(ctas, planes);
-            conv3_wgrad_slab_kernel<CIN, COUT><<<slab_ctas, kConvThreads, 1024u + slab.slots * slab.slot_bytes, st>>>(xm, ym, slab);
+            conv3_wgrad_slab_kernel<CIN, COUT><<<slab_ctas, kConvThreads, 1024u + slab.slots * slab.slot_bytes, st>>>(xs_map, dys_map, slab);
             if (check_launch() != XS_OK) return XS_CUDA_ERROR;
-            wgrad_reduce_kernel<<<(count + 255) / 256, 256, 0, st>>>(partial, slab_ctas, count, dw, accumulate ? 1 : 0);
+            args.redo = slab.redo;
+            args.redo_count = slab_ctas;
+            args.ticket = slab.ticket;
+            // (in place of wgrad_reduce_kernel, both launches together: 16 -> 16 at
+            // 64^3 23.7 -> 22.8 us, 32 -> 32 at 8 x 32^3 27.1 -> 29.1)
+            conv3_wgrad_kernel<CIN, COUT><<<dim3(ctas, L::sets), kConvThreads, L::total, st>>>(xm, ym, args);
             return check_launch();
         }
     }
-    WgradArgs args{s, bx, by, bz, tiles, partial, error};
     conv3_wgrad_kernel<CIN, COUT><<<dim3(ctas, L::sets), kConvThreads, L::total, st>>>(xm, ym, args);
     if (check_launch() != XS_OK) return XS_CUDA_ERROR;
     wgrad_reduce_kernel<<<(count + 255) / 256, 256, 0, st>>>(partial, ctas, count, dw, accumulate ? 1 : 0);

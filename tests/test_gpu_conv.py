@@ -133,6 +133,41 @@ def test_conv_from_halo_slabs(cuda, cout, shape, batch):
         assert bool(((one.float() - out.float()).abs() <= 2.0 ** -7 * one.float().abs() + 1e-4).all())
 
 
+@pytest.mark.parametrize("cin,cout,shape,batch", [(16, 16, (32, 32, 32), 1), (16, 32, (64, 30, 18), 1), (32, 32, (16, 24, 50), 2),
+                                                  (16, 16, (8, 16, 30), 8), (16, 16, (16, 16, 8), 2)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")], ids=["inf", "nan"])
+def test_conv_weight_gradient_of_values_that_are_not_finite(cuda, cin, cout, shape, batch, value):
+    """A voxel of the input that is infinite or NaN reaches the taps that pair
+    it with an output gradient, and no other: voxels in the corners, on the
+    faces and inside, from slabs and (the last shape) from boxes."""
+    import torch
+    from diff_solver_b200 import _native as N
+    L = N.lib()
+    nx, ny, nz = shape
+    g = torch.Generator(device="cpu").manual_seed(11)
+    clean = torch.randn(batch, nz, ny, nx, cin, generator=g).to(torch.bfloat16).cuda()
+    dy = torch.randn(batch, nz, ny, nx, cout, generator=g).to(torch.bfloat16).cuda()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    scratch = torch.full((L.xs_conv3d_weight_grad_scratch_floats(batch, nx, ny, nz, cin, cout),), float("nan"), device="cuda")
+    for z, y, x in ((0, 0, 0), (nz - 1, ny - 1, nx - 1), (nz // 2, ny // 2, nx - 1), (nz // 2, 0, nx // 2), (0, ny // 2, nx // 2),
+                    (nz - 1, ny // 3, 0), (nz // 2, ny // 2, nx // 2), (nz // 2, ny // 2, 0)):
+        xd = clean.clone()
+        xd[batch - 1, z, y, x, 5] = value
+        padded = torch.nn.functional.pad(xd.double(), (0, 0, 1, 1, 1, 1, 1, 1))
+        want = torch.stack([torch.einsum("bzyxi,bzyxo->oi", padded[:, dz:dz + nz, ddy:ddy + ny, dx:dx + nx], dy.double())
+                            for dz, ddy, dx in itertools.product(range(3), repeat=3)])
+        dw = torch.zeros((27, cout, cin), dtype=torch.float32, device="cuda")
+        N.check("wgrad", L.xs_conv3d_weight_grad_bf16(None, batch, nx, ny, nz, cin, cout, xd.data_ptr(), dy.data_ptr(), scratch.data_ptr(),
+                                                      dw.data_ptr(), 0, err.data_ptr()))
+        torch.cuda.synchronize()
+        assert int(err.item()) == 0
+        finite = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(dw), finite), (z, y, x)
+        assert torch.equal(torch.isnan(dw), torch.isnan(want)) and torch.equal(dw[torch.isinf(want)].double(), want[torch.isinf(want)])
+        # (FP64 sums of the same products: as in the test below)
+        assert float((dw.double() - want)[finite].norm() / want[finite].norm()) < 1e-5
+
+
 @pytest.mark.parametrize("cin,cout,shape,batch", [
     (16, 16, (64, 48, 40), 1), (16, 16, (16, 24, 131), 2), (16, 32, (32, 36, 30), 3), (32, 16, (64, 26, 31), 2), (32, 32, (128, 37, 22), 1),
     (16, 16, (4, 64, 100), 4), (32, 32, (8, 48, 140), 2), (16, 16, (256, 21, 19), 1), (16, 16, (128, 800, 1), 1),
