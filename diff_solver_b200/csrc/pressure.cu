@@ -2449,22 +2449,31 @@ XsStatus start_residual(cudaStream_t st, const Grid& g, uint32_t anchor, const u
 // 146x100x56), about what the second would take.
 constexpr uint64_t kDirectTwice = 1200000;
 
+// r = rhs - A x for an almost exact x of a system that the direct solve takes:
+// the rounding of A x in FP32 would drown it.
+template <class T>
+XsStatus direct_residual(cudaStream_t st, const Grid& g, const XsScalarBoundary& pb, const T* rhs, const float* x, float* r) {
+    const uint64_t n = cell_count(g);
+    const uint32_t none = static_cast<uint32_t>(n);  // no anchor cell
+    if (fast_pass_ok(g, nullptr, none, pb, false)) {
+        fast_residual64_kernel<T><<<fast_pass_blocks(g), 256, 0, st>>>(fast_geom(g, none, pb), x, rhs, r);
+    } else {
+        const Operator op{g, nullptr, none, pb, false};
+        start_residual_kernel<T><<<static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 148 * 16)), 256, 0, st>>>(op, rhs, x, r);
+    }
+    return check_launch();
+}
+
+template XsStatus direct_residual<float>(cudaStream_t, const Grid&, const XsScalarBoundary&, const float*, const float*, float*);
+
 template <class T>
 XsStatus direct_start(cudaStream_t st, const Grid& g, const XsScalarBoundary& pb, const WarmHistory& h, const DirectPlan& plan, const T* rhs,
                       const float** guess, float** low) {
     XsStatus s = direct_solve<T>(st, g, plan, rhs, h.extra_product, h.correction, h.ring_start, h.direct);
     *guess = h.ring_start;
     *low = nullptr;
-    const uint64_t n = cell_count(g);
-    if (s != XS_OK || n < kDirectTwice) return s;
-    const uint32_t none = static_cast<uint32_t>(n);  // no anchor cell
-    if (fast_pass_ok(g, nullptr, none, pb, false)) {
-        fast_residual64_kernel<T><<<fast_pass_blocks(g), 256, 0, st>>>(fast_geom(g, none, pb), h.ring_start, rhs, h.residual);
-    } else {
-        const Operator op{g, nullptr, none, pb, false};
-        start_residual_kernel<T><<<static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 148 * 16)), 256, 0, st>>>(op, rhs, h.ring_start, h.residual);
-    }
-    if ((s = check_launch()) != XS_OK) return s;
+    if (s != XS_OK || cell_count(g) < kDirectTwice) return s;
+    if ((s = direct_residual<T>(st, g, pb, rhs, h.ring_start, h.residual)) != XS_OK) return s;
     *low = h.start;
     return direct_solve<float>(st, g, plan, h.residual, h.extra_product, h.correction, h.start, h.direct);
 }

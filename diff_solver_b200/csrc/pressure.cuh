@@ -163,6 +163,9 @@ bool spectral_axes(const Grid& c, const XsScalarBoundary& pb, uint32_t anchor, S
 // x = A^-1 rhs on grid c by the axes' eigenbases (built into basis /
 // eigen: 6 kSpectralMax^2 and 3 kSpectralMax floats).
 XsStatus spectral_solve(cudaStream_t st, const Grid& c, const SpectralAxes& ax, float* basis, float* eigen, const double* rhs, float* x);
+// r = rhs - A x, the products in FP64.
+template <class T>
+XsStatus direct_residual(cudaStream_t st, const Grid& g, const XsScalarBoundary& pb, const T* rhs, const float* x, float* r);
 // The start of a warm-started solve by it: the solution of A x = rhs in two
 // parts, *guess and, on grids past kDirectTwice cells, *low (else null), in
 // h.ring_start and h.start.  h.residual: the residual of the first part

@@ -63,9 +63,7 @@ XsStatus projection_forward(cudaStream_t st, const Grid& g, const XsPressureSolv
         if (warm_start) {
             // the residual of both parts is the first part's less A low
             const float *b = low ? h.residual : rhs, *y = low ? low : x;
-            XsScalarBoundary plain = pb;
-            for (float& v : plain.values) v = 0.0f;
-            if ((s = start_residual(st, g, anchor, mask, plain, b, y, h.correction)) != XS_OK) return s;
+            if ((s = direct_residual(st, g, pb, b, y, h.correction)) != XS_OK) return s;
             if ((s = warm_start_guess(warm_start, st, g, h.correction, &guess)) != XS_OK) return s;
             float* to = low ? low : h.start;
             if ((s = line_step(st, g, anchor, mask, pb, h, guess, y, h.correction, to, false)) != XS_OK) return s;

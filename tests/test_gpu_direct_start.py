@@ -57,6 +57,25 @@ def context(cfg, seed):
             fill_parameters(m.allocate_parameters(ctx), 0.0, -0.1, 0.5))
 
 
+def relative_residual(p, b, res, modes):
+    """|b - A p| / |b| in FP64 (fixed values are 0 in these cases)."""
+    f = np.asarray(p, np.float64).reshape(res[::-1])
+    out = np.zeros_like(f)
+    for d in range(3):
+        axis = 2 - d
+        g = np.moveaxis(f, axis, 0)
+        o = np.moveaxis(out, axis, 0)
+        o[:-1] += g[:-1] - g[1:]
+        o[1:] += g[1:] - g[:-1]
+        if modes[2 * d] == P:
+            o[0] += g[0] - g[-1]
+            o[-1] += g[-1] - g[0]
+        else:
+            o[0] += g[0] if modes[2 * d] == F else 0.0
+            o[-1] += g[-1] if modes[2 * d + 1] == F else 0.0
+    return float(np.linalg.norm(b - out.reshape(-1)) / np.linalg.norm(b))
+
+
 @pytest.mark.parametrize("res,coarsening,modes", CASES, ids=["x".join(map(str, r)) for r, _, _ in CASES])
 def test_start_solves_the_system(cuda, res, coarsening, modes):
     from diff_solver_b200.model import tensors_of
@@ -66,16 +85,25 @@ def test_start_solves_the_system(cuda, res, coarsening, modes):
         nxt, cache = m.allocate_state(ctx), m.allocate_step_cache(ctx)
         m.forward_step(state, control, par, nxt, cache, ctx)
         forward = ctx.read_solve_stats()
+        pressure, rhs = (t.double().cpu().numpy() for t in ctx.pressure_fields())
         seed, prev = m.allocate_state_adjoint(ctx), m.allocate_state_adjoint(ctx)
         for t, s in zip(seed.velocity.components(), state.velocity.components()):
             t.copy_(s)
         m.vjp_step(state, control, par, nxt, cache, seed, prev, m.allocate_control_adjoint(ctx), m.allocate_parameter_adjoint(ctx), ctx)
         adjoint = ctx.read_solve_stats()
         out[warm] = ([t.cpu().numpy() for t in tensors_of(nxt)], [t.cpu().numpy() for t in prev.velocity.components()], forward, adjoint)
-    # FP32 transforms and tridiagonal sweeps: some tens of roundings of x, whose
-    # norm is at most (2 max(res) / pi)^2 times b's, moved by an operator of norm 12
-    part = 12 * 32 * 2.0 ** -24 * (2 * max(res) / np.pi) ** 2
-    bound = min(part, 0.05) ** (2 if n >= 1200000 else 1)
+    # one part: FP32 transforms and tridiagonal sweeps, some tens of roundings of
+    # x, whose norm is at most (2 max(res) / pi)^2 times b's, moved by an operator
+    # of norm 12; on these states it is far from that most, 6e-7 measured.  Two
+    # parts: the second takes the first's residual down as far again
+    # (2e-12 measured), further than any one FP32 vector can (the FP32 rounding
+    # of the solution: 4e-8)
+    part = min(12 * 32 * 2.0 ** -24 * (2 * max(res) / np.pi) ** 2, 1e-5)
+    twice = n >= 1200000
+    bound = 1e-9 if twice else part
+    if twice:
+        assert relative_residual(pressure, rhs, res, modes) > 10 * bound
+        assert all(s["iterations"] == 0 for s in out[True][2:])
     for stats in out[True][2:]:
         assert stats["status"] == 0 and stats["warm_start_used"] == 1 and stats["coarse_iterations"] == 0
         assert stats["initial_residual"] <= bound, (stats["initial_residual"], bound)
@@ -86,6 +114,45 @@ def test_start_solves_the_system(cuda, res, coarsening, modes):
     for a, b in zip(out[True][0] + out[True][1], out[False][0] + out[False][1]):
         if np.linalg.norm(b) > 0:
             assert rel_l2(a, b) < 1e-4, rel_l2(a, b)
+
+
+def test_the_network_works_on_the_residual_of_the_start(cuda):
+    """The residual an almost exact start leaves is formed in FP64 before the
+    network's step: with an FP32 A x most of it is that product's rounding.
+    The trained network at factor 1 then leaves 0.14 of the start's residual
+    (0.24 with FP32 products)."""
+    import os
+    import torch
+    from common import ROOT
+    from diff_solver_b200.data import plume_configuration
+    from diff_solver_b200.model import ExecutionMode, Model, fill_parameters
+    from diff_solver_b200.warm_start import WarmStartNetwork
+    res = (128, 64, 32)
+    cfg = plume_configuration(res)
+    cfg.warm_start_history, cfg.warm_start_coarsening = 5, 2
+    net = WarmStartNetwork(res, factor=1)
+    net.load(os.path.join(ROOT, "diff_solver_b200", "weights", "warm_start_128.npz"))
+    left = []
+    for network in (None, net):
+        m = Model(cfg)
+        ctx = m.allocate_context(ExecutionMode.forward)
+        if network is not None:
+            ctx.set_learned_warm_start(network)
+        s, n = m.allocate_state(ctx), m.allocate_state(ctx)
+        c, k = m.allocate_control(ctx), m.allocate_step_cache(ctx)
+        q = fill_parameters(m.allocate_parameters(ctx), 0.0, -0.1, 0.5)
+        g = torch.Generator().manual_seed(0)
+        for t in s.velocity.components():
+            t.copy_((torch.rand(t.shape, generator=g) * 0.02 - 0.01).cuda())
+        initial = []
+        for _ in range(30):
+            m.forward_step(s, c, q, n, k, ctx)
+            s, n = n, s
+            initial.append(ctx.read_solve_stats()["initial_residual"])
+        left.append(np.mean(initial[10:]))
+    net.check()
+    print(left)
+    assert left[1] < 0.18 * left[0], left
 
 
 def test_settings_keep_the_rounds(cuda):
