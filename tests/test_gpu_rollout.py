@@ -10,11 +10,13 @@
   residual: about 3e-6 relative at 64^3, 1e-5 at 128^3).  Density, temperature and
   velocity must agree to 1e-5 relative L2.
   Where the reference harness is not built (oracle/_ref), against the oracle
-  alone.  Run with the plain zero start, the classical warm start (ring of previous
-  solutions, coarse-grid step) and the benchmark's learned pipeline.
-* The 256^3 headline pipeline (float4 fast paths, three-level coarse start,
-  network step, smoothed PCG): one step after a 30-step rollout against the
-  FP64 oracle's step from the same state.
+  alone.  Run with the plain zero start, the direct start, the ring of previous
+  solutions with rounds of sweeps and coarse-grid steps, and the network's step
+  after either.
+* The 256^3 headline pipeline: one step after a 30-step rollout against the
+  FP64 oracle's step from the same state, from the direct start in two parts
+  and from one round (float4 fast paths, FP32 sweeps, exact coarse solve), each
+  with the network's step after it.
 
 Measured errors are appended to $XS_PARITY_REPORT when it is set.
 """
@@ -67,19 +69,23 @@ def rollout_context(cfg, learned, factor=2):
     return model, ctx, network, params, control, state
 
 
-# (grid, start, steps, check every): the plain zero start; the classical
-# warm start (ring of previous solutions + coarse-grid step); the full
-# learned pipeline (the network runs at factor 1 on 128^3: on a 32^3 network
-# grid its coarsest level is smaller than one convolution tile).
-ROLLOUTS = [(64, "plain", 100, 10), (64, "history+coarse", 100, 10), (128, "learned+history+coarse", 30, 10)]
+# (grid, start, rounds, steps, check every): the plain zero start; the start of
+# the coarse-grid option (rounds = 0: the direct solve of the plume's operator;
+# else ring of previous solutions, sweeps and coarse-grid steps); the network
+# after either (at factor 1 on 128^3: on a 32^3 network grid its coarsest level
+# is smaller than one convolution tile).
+ROLLOUTS = [(64, "plain", 0, 100, 10), (64, "history+coarse", 0, 100, 10), (64, "history+coarse", 2, 100, 10),
+            (128, "learned+history+coarse", 0, 30, 10), (128, "learned+history+coarse", 1, 30, 10)]
 
 
-@pytest.mark.parametrize("n,start,steps,every", ROLLOUTS)
-def test_plume_rollout_matches_oracle_and_reference_kernels(cuda, n, start, steps, every):
+@pytest.mark.parametrize("n,start,rounds,steps,every", ROLLOUTS)
+def test_plume_rollout_matches_oracle_and_reference_kernels(cuda, n, start, rounds, steps, every):
     import torch
     warm = start != "plain"
     learned = start.startswith("learned")
     cfg = plume(n, history=5 if warm else 0, coarsening=2 if warm else 0)
+    cfg.warm_start_rounds = rounds
+    start += f"_rounds{rounds}" if rounds else ""
     model, ctx, network, params, control, cur = rollout_context(cfg, learned=learned, factor=1 if n <= 128 else 4)
     nxt = model.allocate_state(ctx)
     cache = model.allocate_step_cache(ctx)
@@ -121,9 +127,11 @@ def test_plume_rollout_matches_oracle_and_reference_kernels(cuda, n, start, step
     report(f"rollout{n}_{start}_worst", **worst)
 
 
-def test_headline_pipeline_step_at_256_matches_fp64_oracle(cuda):
+@pytest.mark.parametrize("rounds", [0, 1])
+def test_headline_pipeline_step_at_256_matches_fp64_oracle(cuda, rounds):
     import torch
     cfg = plume(256, history=5, coarsening=2)
+    cfg.warm_start_rounds = rounds
     # the benchmark's network: trained at 128^3, run on the grid restricted x4
     model, ctx, network, params, control, cur = rollout_context(cfg, learned=True, factor=4)
     nxt = model.allocate_state(ctx)

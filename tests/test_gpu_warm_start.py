@@ -262,18 +262,60 @@ def test_adjoint_solves_start_from_their_own_history(cuda):
     assert out[(4, 4)][2] == 0 and out[(4, 4)][1] < out[(4, 0)][1], (out[(4, 4)][1:], out[(4, 0)][1:])
 
 
-def test_coarse_grid_correction(cuda):
+def test_adjoint_rounds_over_an_exactly_solved_coarse_grid(cuda):
+    """Adjoint solves have no setting of their own: their three rounds over an
+    exactly solved coarse grid serve operators that separate but have two axes
+    with unequal ends, which the direct start does not take.  Same gradient,
+    fewer iterations than the ring alone, none on the coarse grid."""
+    import torch
+    from diff_solver_b200.data import ScalarBoundaryMode, VelocityBoundaryMode, plume_configuration
+    from diff_solver_b200.model import ExecutionMode, Model, fill_parameters
+    from diff_solver_b200.solver import TapeMode, simulate, vjp
+    out = {}
+    for history, coarsening in ((0, 0), (4, 0), (4, 2)):
+        cfg = plume_configuration((48, 64, 40))
+        cfg.velocity_boundary.x_max.mode = VelocityBoundaryMode.zero_gradient
+        cfg.pressure_boundary.x_max.mode = ScalarBoundaryMode.fixed_value
+        cfg.pressure_boundary.x_max.value = 0.0
+        cfg.warm_start_history, cfg.warm_start_coarsening = history, coarsening
+        m = Model(cfg)
+        ctx = m.allocate_context(ExecutionMode.differentiable)
+        q = fill_parameters(m.allocate_parameters(ctx), 0.0, -0.1, 0.5)
+        controls = [m.allocate_control(ctx) for _ in range(10)]
+        s0 = m.allocate_state(ctx)
+        g = torch.Generator().manual_seed(0)
+        for t in s0.velocity.components():
+            t.copy_((torch.rand(t.shape, generator=g) * 0.02 - 0.01).cuda())
+        traj = simulate(m, ctx, s0, controls, q, TapeMode.store_all)
+        forward = ctx.read_solve_stats()
+        seed = m.allocate_state_adjoint(ctx)
+        seed.density.values.copy_(traj.states[-1].density.values.double())
+        grad = vjp(m, ctx, traj, controls, q, {10: seed})
+        last = ctx.read_solve_stats()
+        for st in (forward, last):
+            assert st["status"] == 0 and st["final_residual"] <= 1e-6 and st["coarse_iterations"] == 0
+        out[(history, coarsening)] = (torch.cat([t.reshape(-1) for t in grad.initial_state.velocity.components()]).cpu().numpy(),
+                                      last["iterations"], last["initial_residual"])
+    print({k: v[1:] for k, v in out.items()})
+    assert rel(out[(4, 0)][0], out[(0, 0)][0]) < 1e-3 and rel(out[(4, 2)][0], out[(0, 0)][0]) < 1e-3
+    # the rounds leave iterations to do: not the direct start
+    assert 0 < out[(4, 2)][1] < out[(4, 0)][1] <= out[(0, 0)][1], {k: v[1:] for k, v in out.items()}
+
+
+@pytest.mark.parametrize("rounds", [0, 2])
+def test_coarse_grid_correction(cuda, rounds):
     """The coarse-grid correction of the history start: the same steps within
     the solver tolerance and far fewer fine iterations than the history start
     alone once the plume has developed (the smooth error the correction
     removes is what keeps CG on its residual plateau).  The plume's operator
     separates (open top, no anchor): its coarse grid is solved exactly and
-    reports no coarse CG iterations."""
+    reports no coarse CG iterations (rounds = 0: the fine grid's is, at once)."""
     from diff_solver_b200.data import plume_configuration
     cfg = plume_configuration((128, 128, 128))
     cfg.warm_start_history = 5
     hist, hist_stats, _ = _rollout(cfg, 50)
     cfg.warm_start_coarsening = 4
+    cfg.warm_start_rounds = rounds
     coarse, coarse_stats, _ = _rollout(cfg, 50)
     assert all(s["status"] == 0 and s["final_residual"] <= 1e-6 for s in coarse_stats)
     assert rel(coarse, hist) < 1e-4
@@ -284,17 +326,19 @@ def test_coarse_grid_correction(cuda):
     assert late_coarse < 0.7 * late_hist, (late_coarse, late_hist)
 
 
-def test_coarse_grid_correction_on_axes_past_128(cuda):
+@pytest.mark.parametrize("rounds", [0, 2])
+def test_coarse_grid_correction_on_axes_past_128(cuda, rounds):
     """A coarse axis of 129-256 cells (the case of the 512x512x256 plume,
     here 320 x 96 x 64 coarsened x2 to 160 x 48 x 32) is solved exactly as
     well, by the transforms that take the basis in two halves: converged
     steps, the history start's steps within the tolerance, no coarse CG
-    iterations, fewer fine iterations."""
+    iterations, fewer fine iterations (rounds = 0: the fine grid at once)."""
     from diff_solver_b200.data import plume_configuration
     cfg = plume_configuration((320, 96, 64), inflow_center=(0.5, 0.05, 0.1), inflow_radius=0.04)
     cfg.warm_start_history = 5
     hist, hist_stats, _ = _rollout(cfg, 30)
     cfg.warm_start_coarsening = 2
+    cfg.warm_start_rounds = rounds
     coarse, coarse_stats, _ = _rollout(cfg, 30)
     assert all(s["status"] == 0 and s["final_residual"] <= 1e-6 for s in coarse_stats)
     assert rel(coarse, hist) < 1e-4
@@ -327,9 +371,11 @@ def test_coarse_grid_correction_by_coarse_cg(cuda):
     assert late_coarse < late_hist, (late_coarse, late_hist)
 
 
-def test_coarse_correction_with_learned_guess(cuda):
+@pytest.mark.parametrize("rounds", [0, 1])
+def test_coarse_correction_with_learned_guess(cuda, rounds):
     """Ring start, coarse-grid step, then the network's step on the residual
-    left by that: converged, same steps."""
+    left by that (rounds = 0: the network's step after the direct start):
+    converged, same steps."""
     from diff_solver_b200.data import plume_configuration
     from diff_solver_b200.warm_start import WarmStartNetwork
     res = (128, 64, 32)
@@ -337,6 +383,7 @@ def test_coarse_correction_with_learned_guess(cuda):
     plain, _, _ = _rollout(cfg, 8)
     cfg.warm_start_history = 5
     cfg.warm_start_coarsening = 2
+    cfg.warm_start_rounds = rounds
     net = WarmStartNetwork(res, factor=1, seed=4)
     warm, warm_stats, _ = _rollout(cfg, 8, network=net)
     net.check()
