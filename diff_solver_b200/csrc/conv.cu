@@ -217,16 +217,14 @@ __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __gri
 // more than another start address: (dy (X + 2) + dx) voxels into plane dz.  A
 // tile's 128 rows are consecutive voxels of the widened rows; the two columns
 // between rows are computed too and dropped (at X = 64 and 11 rows 92 % of the
-// products are kept).  The weights are loaded one tap per stage of a ring that
-// holds all 27 of the narrowest layers.
+// products are kept).  The weights of all 27 taps lie beside it, a barrier each.
 //
 // What bounds it is the rate at which one warp issues 128 x 16 x 16 MMAs, 40
-// cycles each from uniform registers: 16 -> 16 at 64^3 runs in 23 us (the
-// shifted boxes, 27 x 8.4 MB through L2: 46 to 50), 8 x 64^3 in 153 (294), of
+// cycles each from uniform registers: 16 -> 16 at 64^3 runs in 23.5 us (the
+// shifted boxes, 27 x 8.4 MB through L2: 48.6), 8 x 64^3 in 148 (332), of
 // which the MMAs are 70.  The unswizzled layout, 8 voxels by 16 bytes at a
 // time, gives the same numbers at a quarter of the operand rate: 140 cycles
 // per MMA.
-//
 constexpr int kSlabThreads = 256;
 
 template <int CIN, int COUT>
@@ -234,10 +232,8 @@ struct SlabSmem {
     static constexpr uint32_t chunks = CIN / 8;
     static constexpr uint32_t w_bytes_raw = static_cast<uint32_t>(COUT) * CIN * 2u;
     static constexpr uint32_t w_bytes = (w_bytes_raw + 1023u) / 1024u * 1024u;
-    // as many taps as 96 KB hold, all 27 but for the widest layers: a stage
-    // filled again costs the MMAs' completion and a load's latency
-    static constexpr int ring = 98304u / w_bytes < 27u ? static_cast<int>(98304u / w_bytes) : 27;
-    static constexpr uint32_t fixed = 1024u /*alignment*/ + ring * w_bytes + 512u /*barriers*/;
+    static constexpr uint32_t fixed = 1024u /*alignment*/ + 27u * w_bytes + 512u /*barriers*/;
+    static_assert(CIN == 16 && 27u * w_bytes <= 98304u);  // one MMA of K = 16 per tap and tile; room for a box
 };
 constexpr uint32_t kSlabMaxSmem = 220u * 1024u;
 constexpr uint64_t kSlabMinVoxels = 100000u;
@@ -264,12 +260,11 @@ template <int CIN, int COUT>
 __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ SlabArgs a) {
     using L = SlabSmem<CIN, COUT>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    unsigned char* w_ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
-    uint64_t* full = reinterpret_cast<uint64_t*>(w_ring + L::ring * L::w_bytes);
-    uint64_t* empty = full + L::ring;
-    uint64_t* accum = empty + L::ring;
+    unsigned char* taps = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
+    uint64_t* full = reinterpret_cast<uint64_t*>(taps + 27u * L::w_bytes);
+    uint64_t* accum = full + 27;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(accum + 1);
-    unsigned char* slab = w_ring + L::ring * L::w_bytes + 512;
+    unsigned char* slab = taps + 27u * L::w_bytes + 512;
     const int warp = static_cast<int>(tc::uniform(threadIdx.x >> 5)), lane = threadIdx.x & 31;
     const uint32_t strips = (a.s.y + a.p.by - 1) / a.p.by, layers = (a.s.z + a.p.bz - 1) / a.p.bz;
     const uint32_t strip = blockIdx.x % strips, layer = blockIdx.x / strips % layers, b = blockIdx.x / strips / layers;
@@ -280,10 +275,7 @@ __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_c
     const uint32_t plane_bytes = a.p.voxels * row_bytes;
 
     if (threadIdx.x == 0) {
-        for (int i = 0; i < L::ring; ++i) {
-            tc::mbar_init(&full[i], 1);
-            tc::mbar_init(&empty[i], 1);
-        }
+        for (int i = 0; i < 27; ++i) tc::mbar_init(&full[i], 1);
         tc::mbar_init(accum, 1);
         tc::fence_barrier_init();
         tc::prefetch_map(&w_map);
@@ -293,12 +285,12 @@ __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_c
         tc::tmem_relinquish();
     }
     __syncthreads();
-    auto load_weights = [&](int tap) {
-        tc::mbar_expect_tx(&full[tap % L::ring], L::w_bytes_raw);
-        tc::tma_load_3d(w_ring + (tap % L::ring) * L::w_bytes, &w_map, &full[tap % L::ring], 0, 0, tap);
-    };
-    if (warp == 0 && tc::elect_one())
-        for (int tap = 0; tap < L::ring; ++tap) load_weights(tap);
+    if (warp == 0 && tc::elect_one()) {
+        for (int tap = 0; tap < 27; ++tap) {
+            tc::mbar_expect_tx(&full[tap], L::w_bytes_raw);
+            tc::tma_load_3d(taps + tap * L::w_bytes, &w_map, &full[tap], 0, 0, tap);
+        }
+    }
     __syncwarp();
     // the box, zeros beyond the volume: a warp per row, 16 bytes per lane
     for (int r = warp; r < (planes + 2) * (rows + 2); r += kSlabThreads / 32) {
@@ -323,47 +315,34 @@ __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_c
     tc::tc_fence_after();
     const uint32_t tmem = tc::uniform(*tmem_slot);
     bool ok = true;
-    if (warp == 0) {
-        // the taps past the ring
-        if (L::ring < 27 && tc::elect_one()) {
-            for (int tap = L::ring; tap < 27; ++tap) {
-                if (!tc::mbar_wait(&empty[tap % L::ring], (tap / L::ring - 1) & 1)) { ok = false; break; }
-                load_weights(tap);
-            }
-        }
-    } else if (warp == 1) {
+    if (warp == 1) {
         constexpr uint32_t idesc = tc::idesc_bf16(128, COUT, false, false);
-        constexpr uint32_t w_row = CIN * 2;
-        // descriptors of the box and of the ring; steps in their 16-byte units
+        // descriptors of the box and of the taps; steps in their 16-byte units
         const uint64_t box = tc::smem_desc(tc::uniform(tc::smem_u32(slab)), 16u, 8u * row_bytes, tc::swizzle_for_row_bytes(row_bytes));
-        const uint64_t weights = tc::smem_desc(tc::uniform(tc::smem_u32(w_ring)), 16u, 8u * w_row, tc::swizzle_for_row_bytes(w_row));
+        const uint64_t weights = tc::smem_desc(tc::uniform(tc::smem_u32(taps)), 16u, 8u * row_bytes, tc::swizzle_for_row_bytes(row_bytes));
         constexpr uint32_t tile_step = 128u * row_bytes / 16u;
         const uint32_t plane_step = plane_bytes / 16u, tiles = a.p.tiles;
         if (tc::elect_one()) {
-            uint32_t accumulate = 0u;
             for (int tap = 0; tap < 27; ++tap) {
-                const int s = tap % L::ring, round = tap / L::ring;
-                if (!tc::mbar_wait(&full[s], round & 1)) { ok = false; break; }
+                if (!tc::mbar_wait(&full[tap], 0)) { ok = false; break; }
                 tc::tc_fence_after();
                 const uint32_t dz = static_cast<uint32_t>(tap) / 9u, dy = static_cast<uint32_t>(tap) / 3u % 3u, dx = static_cast<uint32_t>(tap) % 3u;
-                const uint64_t from = box + dz * plane_step + (dy * px + dx) * (row_bytes / 16u), w = weights + s * (L::w_bytes / 16u);
-#pragma unroll
-                for (uint32_t k = 0; k < CIN / 16; ++k) {
-                    uint32_t d = tmem;
-                    uint64_t plane = from + 2u * k;
-                    for (int z = 0; z < planes; ++z) {
-                        uint64_t tile = plane;
+                const uint64_t w = weights + tap * (L::w_bytes / 16u);
+                uint64_t plane = box + dz * plane_step + (dy * px + dx) * (row_bytes / 16u);
+                uint32_t d = tmem;
+                for (int z = 0; z < planes; ++z) {
+                    uint64_t tile = plane;
 #pragma unroll 4
-                        for (uint32_t t = 0; t < tiles; ++t) {
-                            tc::mma_bf16(d, tile, w + 2u * k, idesc, accumulate);
-                            tile += tile_step;
-                            d += COUT;
-                        }
-                        plane += plane_step;
+                    for (uint32_t t = 0; t < tiles; ++t) {
+                        tc::mma_bf16(d, tile, w, idesc, tap > 0 ? 1u : 0u);
+                        tile += tile_step;
+                        d += COUT;
                     }
-                    accumulate = 1u;
+                    plane += plane_step;
                 }
-                tc::mma_commit(&empty[s]);
+                // (nothing waits for it: CTAs that share an SM's tensor pipe take
+                // turns tap by tap; 16 -> 64 at 128^3 307 us, 327 without)
+                tc::mma_commit(&full[tap]);
             }
             tc::mma_commit(accum);
         }
@@ -407,9 +386,13 @@ __global__ void __launch_bounds__(kSlabThreads) conv3_slab_kernel(const __grid_c
 // to 174 strips of 16 -> 16 at 64^3, 8 x 64^3, 128^3 and 128 x 128 x 64: a wave
 // of r CTAs per SM (by shared memory and TMEM) costs 10 us for the box, the
 // launch and the epilogue, and per MMA of a CTA 20 ns and 11 ns more for each of
-// the r that share the tensor pipe.  Its picks take 23.0, 152.7, 158.1 and
+// the r that share the tensor pipe.  Its picks took 23.0, 152.7, 158.1 and
 // 89.6 us; the best strips 23.0, 143.0, 158.1 and 89.6.  (Counting the parts of
-// one CTA in cycles picked 26.9, 158.5, 158.2 and 98.6.)
+// one CTA in cycles picked 26.9, 158.5, 158.2 and 98.6.)  The constants serve
+// 16 -> 32 and 16 -> 64 unfitted, whose MMAs take longer: against the boxes 64^3
+// 30.4 (50.8) and 50.8 (65.6), 128^3 219 (344) and 308 (463), 8 x 64^3 162 (345)
+// and 345 (463).  Of 13 shapes of 131,072 voxels and more the boxes are faster in
+// one, 16 -> 64 at 8 x 16 x 1024 (37.3 against 39.1): rows of 8 in rows of 10.
 template <int CIN, int COUT>
 bool slab_plan(const VolumeShape& s, SlabPlan& best) {
     using L = SlabSmem<CIN, COUT>;
@@ -460,8 +443,8 @@ XsStatus launch_conv_forward(cudaStream_t st, const VolumeShape& s, const __nv_b
     uint32_t bx, by, bz;
     if (!conv_tile(s, bx, by, bz)) return XS_INVALID_ARGUMENT;
     // The slab wins where the 27 shifted boxes of narrow layers fill the SMs:
-    // 16 -> 16 at 64^3 23 us against 46 from the boxes, at 8 x 64^3 153
-    // against 294; 16 -> 32 at 8 x 32^3 29 against 48.  With fewer voxels a CTA
+    // 16 -> 16 at 64^3 23.5 us against 48.6 from the boxes, at 8 x 64^3 148
+    // against 332; 16 -> 32 at 8 x 32^3 29 against 50.  With fewer voxels a CTA
     // has too few MMAs behind one box to wait for (16 -> 32 at 32^3 14.1 us
     // against 11.1; by both slopes they meet near 100,000 voxels), and from 32
     // channels on a box fills an MMA's time anyway (32 -> 16 at 8 x 32^3 52.0

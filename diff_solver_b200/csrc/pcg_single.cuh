@@ -43,7 +43,6 @@ struct PadGeom {
     uint32_t nx, ny, nz, n;
     uint32_t pitch, rows, plane, base;
     uint32_t total;  // floats per vector
-    uint32_t quads;  // 4-cell groups from `base`, a whole number of warps
     FastDiv dnx, dny, dpitch, drows;
     uint32_t periodic;  // bit d: axis d wraps
 

@@ -97,7 +97,7 @@ PadExtents pad_extents(const Grid& g, const uint32_t (&modes)[6]) {
     e.pitch = (static_cast<uint64_t>(g.nx) + (wraps(0) ? 2 : 1) + 3) / 4 * 4;
     e.rows = static_cast<uint64_t>(g.ny) + (wraps(1) ? 2 : 1);
     e.plane = e.pitch * e.rows;
-    e.total = e.plane * (static_cast<uint64_t>(g.nz) + 2) + 256;  // a warp's worth past the last plane
+    e.total = e.plane * (static_cast<uint64_t>(g.nz) + 2);
     return e;
 }
 
@@ -1288,7 +1288,6 @@ PadGeom pad_geom(const Grid& g, const XsScalarBoundary& pb) {
     p.plane = static_cast<uint32_t>(e.plane);
     p.base = p.plane;
     p.total = static_cast<uint32_t>(e.total);
-    p.quads = (p.plane / 4u * p.nz + 31u) / 32u * 32u;
     p.dnx = make_fastdiv(p.nx);
     p.dny = make_fastdiv(p.ny);
     p.dpitch = make_fastdiv(p.pitch);
