@@ -13,19 +13,22 @@ The plume first spins up from rest (seeded uniform velocity noise in
 
   plain                   zero start (the reference's zero-initialised solve)
   history                 Galerkin start from the last 5 forward solutions
-  history+coarse          ... then two rounds of Jacobi sweeps and a step along
-                          the coarse-grid correction (coarse grid solved exactly
-                          when its operator separates)
+  history+coarse          with the coarse-grid correction switched on: where the
+                          grid's own operator separates, as the plume's does, a
+                          direct solve of it in FP32 and a second one on the FP64
+                          residual (else two rounds of Jacobi sweeps and a step
+                          along the coarse grid's solution)
   learned                 the warm-start network's guess alone, energy-scaled
   learned+history         the ring start, then a step along the network's
                           correction of its residual
-  learned+history+coarse  the ring start, one round of sweeps and coarse-grid
-                          step, then the network's step (headline)
+  learned+history+coarse  that start, then the network's step (headline)
 
 Each arm runs W warm-up steps (which also refill its ring) and K timed steps,
 every timed step with per-stage CUDA events (XsSmokeModel.stage_events).
-``value`` is the headline arm's steps/s; every arm's steps/s, PCG iterations
-and per-stage times are in ``arms``.  Further records of the same run:
+``value`` is the headline arm's steps/s; ``arms`` has every arm's.  The result is
+one JSON line on stdout, short enough to be read from the end of a log; a second
+one on stderr ({"records": ...}) holds every arm's iterations and per-stage times
+and the further records of the run:
 
   roofline            the headline arm's dominant kernel, the fine PCG launch
                       (stage events around it), against the measured copy peak
@@ -903,6 +906,16 @@ def reference_run(args):
     return cpu_steps(host_state, args.shape, budget_s=args.cpu_budget, max_steps=min(args.steps, args.cpu_steps))
 
 
+RECORDS = ("arms", "roofline_plain", "example_metrics_last_step", "adjoint", "network", "config0", "reference_kernels", "large_grid")
+
+
+def split_result(line):
+    """The result line, with a summary of its arms, and its further records."""
+    short = {k: v for k, v in line.items() if k not in RECORDS}
+    short["arms"] = {name: {k: arm[k] for k in ("steps_per_s", "ms_per_step", "mean_pcg_iterations")} for name, arm in line["arms"].items()}
+    return short, {k: line[k] for k in RECORDS if k in line}
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -1029,6 +1042,8 @@ def main():
     if host_state is not None and "plain" in arms:
         cpu = cpu_steps(host_state, args.shape, budget_s=30.0, max_steps=1)
         line["cpu_baseline"] = {k: cpu[k] for k in ("value", "unit", "cores", "kind", "sample")}
+    line, records = split_result(line)
+    print(json.dumps({"records": records}), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
 
 

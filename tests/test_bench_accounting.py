@@ -2,6 +2,7 @@
 byte counts follow the stage table of the smoke step, the U-Net FLOP table
 describes the network the library builds (its parameter count), and the CPU
 oracle leg of the 64^3 record produces its timing record."""
+import json
 import os
 import sys
 
@@ -17,6 +18,18 @@ def test_convolution_table_matches_the_library_network():
     # every convolution holds 27 x C_in x C_out weights (no biases)
     weights = sum(27 * cin * cout for cin, cout, _ in bench.UNET_CONVOLUTIONS)
     assert weights == _native.lib().xs_warm_start_parameter_count() == 525_312
+
+
+def test_result_line_is_short_and_drops_nothing():
+    arm = {"steps_per_s": 1.0, "ms_per_step": 2.0, "mean_pcg_iterations": 3.0, "stages": {k: {"ms": 0.1} for k in bench.STAGES},
+           "pcg_iterations_per_step": list(range(200))}
+    line = {"metric": bench.METRIC, "value": 1.0, "unit": bench.UNIT, "n_gpus": 1, "steps": 20, "warmup": 5, "config": {"grid": [1]},
+            "gpu_launches": 7, "clocks": {}, "e2e": {"value": 1.0}, "arms": {f"arm{i}": arm for i in range(6)}, "adjoint": {"x": [0] * 5000}}
+    short, records = bench.split_result(line)
+    assert len(json.dumps(short)) < 1500
+    assert set(short) | set(records) == set(line) and all(short[k] == line[k] for k in short if k != "arms")
+    assert records["arms"] == line["arms"] and records["adjoint"] == line["adjoint"]
+    assert short["arms"]["arm3"] == {"steps_per_s": 1.0, "ms_per_step": 2.0, "mean_pcg_iterations": 3.0}
 
 
 def test_unet_flops():
