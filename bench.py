@@ -30,8 +30,8 @@ one JSON line on stdout, short enough to be read from the end of a log; a second
 one on stderr ({"records": ...}) holds every arm's iterations and per-stage times
 and the further records of the run:
 
-  roofline            the headline arm's dominant kernel, the fine PCG launch
-                      (stage events around it), against the measured copy peak
+  roofline            the headline arm's fine PCG launch (stage events around
+                      it), against the measured copy peak
   roofline_plain      the same kernel in the plain arm
   adjoint             the 40-step VJP (checkpoints every 8) ending at step 200,
                       with the reverse step's algorithmic bytes

@@ -154,9 +154,11 @@ class Configuration:
     # forward PCG solve (0..5; 0: off)
     warm_start_history: int = 0
     # coarse-grid correction of that start (0: off; else the coarsening
-    # factor per axis, dividing the grid; needs a ring and no colliders)
+    # factor per axis, dividing the grid; needs a ring and no colliders); a
+    # direct solve of the grid itself instead, where its operator separates
     warm_start_coarsening: int = 0
-    # rounds of sweeps and coarse-grid correction before a forward solve (0: defaults)
+    # rounds of sweeps and coarse-grid correction before a forward solve (0:
+    # the defaults, or the direct solve; else rounds on every grid)
     warm_start_rounds: int = 0
 
 

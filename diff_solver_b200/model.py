@@ -181,7 +181,8 @@ class ExecutionContext:
     def warm_start_fields(self):
         """(x0, b - A x0) of the last forward solve, x0 the Galerkin start from
         the ring of previous solutions (configuration.warm_start_history > 0),
-        as device tensors viewing the workspace."""
+        whatever the solve itself started from, as device tensors viewing the
+        workspace."""
         x, r = C.c_void_p(), C.c_void_p()
         N.check("xs_smoke_warm_start_fields", N.lib().xs_smoke_warm_start_fields(self.stream_handle, C.byref(self.native),
                                                                                    C.c_void_p(self.workspace.data_ptr()), C.byref(x),

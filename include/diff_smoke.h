@@ -341,7 +341,7 @@ typedef struct XsSmokeModel {
      * (warm_start_rounds).  It removes the smooth error that fine-grid CG
      * reduces slowest.
      * Where the fluid grid's own operator separates (no anchor cell, no fixed
-     * boundary value other than 0, at most 512 cells per axis, equal ends or
+     * boundary value other than 0, 4 to 512 cells per axis, equal ends or
      * periodic x and y or z, the third axis not periodic) and
      * warm_start_rounds is 0, the system is solved there directly instead, in
      * FP32, and neither ring nor rounds enter the start (the ring is kept for

@@ -94,9 +94,11 @@ struct Configuration {
     // previous forward solutions kept for the Galerkin warm start (0..5; 0: off)
     std::uint32_t warm_start_history{0u};
     // coarse-grid correction of that start (0: off; else the coarsening factor
-    // per axis, dividing the grid; needs a ring and no colliders)
+    // per axis, dividing the grid; needs a ring and no colliders); a direct
+    // solve of the grid itself instead, where its operator separates
     std::uint32_t warm_start_coarsening{0u};
-    // rounds of sweeps and coarse-grid correction before a forward solve (0: defaults)
+    // rounds of sweeps and coarse-grid correction before a forward solve (0:
+    // the defaults, or the direct solve; else rounds on every grid)
     std::uint32_t warm_start_rounds{0u};
 };
 
