@@ -485,8 +485,12 @@ __device__ __forceinline__ uint32_t fastdiv(uint32_t n, const FastDiv& f) {
     return static_cast<uint32_t>((static_cast<uint64_t>(n) * f.m) >> f.shift);
 }
 
+// No neighbour.  (0 is an offset: a periodic row of 4 cells, one group, finds its
+// last cell's neighbour at its own start, a periodic axis of one cell itself.)
+constexpr int32_t kNoCell = INT32_MIN;
+
 struct RowGeom {
-    int32_t off[4];  // -y, +y, -z, +z neighbour offsets; 0 = no neighbour
+    int32_t off[4];  // -y, +y, -z, +z neighbour offsets, or kNoCell
     float dyz;       // diagonal share of the y and z directions
 };
 
@@ -502,25 +506,25 @@ __device__ __forceinline__ RowGeom row_geom(const FastGeom& f, uint32_t y, uint3
         // lower side
         if (c[d] > 0) { r.off[2 * d] = -stride[d]; r.dyz += 1.0f; }
         else if (f.kind[2 + 2 * d] == 2u) { r.off[2 * d] = stride[d] * static_cast<int32_t>(size[d] - 1); r.dyz += 1.0f; }
-        else { r.off[2 * d] = 0; if (f.kind[2 + 2 * d] == 1u) r.dyz += 1.0f; }
+        else { r.off[2 * d] = kNoCell; if (f.kind[2 + 2 * d] == 1u) r.dyz += 1.0f; }
         // upper side
         if (c[d] + 1 < size[d]) { r.off[2 * d + 1] = stride[d]; r.dyz += 1.0f; }
         else if (f.kind[3 + 2 * d] == 2u) { r.off[2 * d + 1] = -stride[d] * static_cast<int32_t>(size[d] - 1); r.dyz += 1.0f; }
-        else { r.off[2 * d + 1] = 0; if (f.kind[3 + 2 * d] == 1u) r.dyz += 1.0f; }
+        else { r.off[2 * d + 1] = kNoCell; if (f.kind[3 + 2 * d] == 1u) r.dyz += 1.0f; }
     }
     return r;
 }
 
-// Offsets of the x neighbours of the group's first and last cell (0: none)
+// Offsets of the x neighbours of the group's first and last cell (or kNoCell)
 // and the diagonals of the four cells.
 __device__ __forceinline__ void x_geom(const FastGeom& f, uint32_t x0, float dyz, int32_t& left, int32_t& right, float4& d) {
     d = make_float4(dyz + 2.0f, dyz + 2.0f, dyz + 2.0f, dyz + 2.0f);
     if (x0 > 0) left = -1;
     else if (f.kind[0] == 2u) left = static_cast<int32_t>(f.nx) - 1;
-    else { left = 0; d.x -= f.kind[0] == 1u ? 0.0f : 1.0f; }
+    else { left = kNoCell; d.x -= f.kind[0] == 1u ? 0.0f : 1.0f; }
     if (x0 + 4 < f.nx) right = 4;
     else if (f.kind[1] == 2u) right = 4 - static_cast<int32_t>(f.nx);
-    else { right = 0; d.w -= f.kind[1] == 1u ? 0.0f : 1.0f; }
+    else { right = kNoCell; d.w -= f.kind[1] == 1u ? 0.0f : 1.0f; }
 }
 
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -576,13 +580,13 @@ __device__ void spmv_fast(const PcgArgs& a, const FastGeom& f, int k, float beta
         float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            if (rg.off[q] != 0) {
+            if (rg.off[q] != kNoCell) {
                 const float4 v = value4(static_cast<uint32_t>(static_cast<int32_t>(i) + rg.off[q]));
                 s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
             }
         }
-        const float l = left != 0 ? value1(static_cast<uint32_t>(static_cast<int32_t>(i) + left)) : 0.0f;
-        const float r = right != 0 ? value1(static_cast<uint32_t>(static_cast<int32_t>(i) + right)) : 0.0f;
+        const float l = left != kNoCell ? value1(static_cast<uint32_t>(static_cast<int32_t>(i) + left)) : 0.0f;
+        const float r = right != kNoCell ? value1(static_cast<uint32_t>(static_cast<int32_t>(i) + right)) : 0.0f;
         float4 qv;
         qv.x = d.x * c.x - (s.x + l + c.y);
         qv.y = d.y * c.y - (s.y + c.x + c.z);
@@ -689,13 +693,13 @@ __device__ __forceinline__ Double4 apply4(const FastGeom& f, const float* __rest
               static_cast<double>(d.w) * c.w};
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        if (rg.off[k] != 0) {
+        if (rg.off[k] != kNoCell) {
             const float4 v = ld4(x + static_cast<uint32_t>(static_cast<int32_t>(i) + rg.off[k]));
             q.x -= v.x; q.y -= v.y; q.z -= v.z; q.w -= v.w;
         }
     }
-    if (left != 0) q.x -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + left)];
-    if (right != 0) q.w -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + right)];
+    if (left != kNoCell) q.x -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + left)];
+    if (right != kNoCell) q.w -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + right)];
     q.x -= c.y;
     q.y -= static_cast<double>(c.x) + c.z;
     q.z -= static_cast<double>(c.y) + c.w;
@@ -718,13 +722,13 @@ __device__ __forceinline__ float4 apply4f(const FastGeom& f, const float* __rest
     float4 q = make_float4(d.x * c.x, d.y * c.y, d.z * c.z, d.w * c.w);
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        if (rg.off[k] != 0) {
+        if (rg.off[k] != kNoCell) {
             const float4 v = ld4(x + static_cast<uint32_t>(static_cast<int32_t>(i) + rg.off[k]));
             q.x -= v.x; q.y -= v.y; q.z -= v.z; q.w -= v.w;
         }
     }
-    if (left != 0) q.x -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + left)];
-    if (right != 0) q.w -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + right)];
+    if (left != kNoCell) q.x -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + left)];
+    if (right != kNoCell) q.w -= x[static_cast<uint32_t>(static_cast<int32_t>(i) + right)];
     q.x -= c.y;
     q.y -= c.x + c.z;
     q.z -= c.y + c.w;
@@ -818,15 +822,15 @@ __device__ __forceinline__ void apply4_fp64(const FastGeom& f, const View& x, ui
     for (int k = 0; k < 4; ++k) ax[k] = static_cast<double>(dd[k]) * c[k];
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-        if (rg.off[q] != 0) {
+        if (rg.off[q] != kNoCell) {
             double v[4];
             load_x4(x, static_cast<uint32_t>(static_cast<int32_t>(i) + rg.off[q]), v);
 #pragma unroll
             for (int k = 0; k < 4; ++k) ax[k] -= v[k];
         }
     }
-    if (left != 0) ax[0] -= static_cast<double>(x[static_cast<uint32_t>(static_cast<int32_t>(i) + left)]);
-    if (right != 0) ax[3] -= static_cast<double>(x[static_cast<uint32_t>(static_cast<int32_t>(i) + right)]);
+    if (left != kNoCell) ax[0] -= static_cast<double>(x[static_cast<uint32_t>(static_cast<int32_t>(i) + left)]);
+    if (right != kNoCell) ax[3] -= static_cast<double>(x[static_cast<uint32_t>(static_cast<int32_t>(i) + right)]);
     ax[0] -= c[1];
     ax[1] -= c[0] + c[2];
     ax[2] -= c[1] + c[3];

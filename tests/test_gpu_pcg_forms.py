@@ -25,6 +25,10 @@ RESIDENT = [
     ((34, 9, 31), (P, P, P, P, Z, F), True), ((35, 12, 11), (P, P, P, P, P, P), False), ((48, 40, 36), (Z,) * 6, True),
     ((64, 64, 64), PLUME, False), ((70, 61, 53), PLUME, True), ((97, 60, 59), (P, P, Z, F, P, P), True), ((90, 88, 75), PLUME, False),
 ]
+# periodic axes of one cell, and periodic rows of 4, whose ends are one group
+WRAPPED = [((4, 7, 5), (P, P, Z, F, Z, Z), False), ((8, 1, 6), (Z, F, P, P, Z, Z), False), ((12, 6, 1), (Z, F, Z, Z, P, P), False),
+           ((4, 1, 9), (P, P, P, P, F, Z), False), ((4, 6, 5), (P, P, P, P, P, P), False), ((4, 128, 96), (P, P, Z, F, Z, Z), False),
+           ((1200, 1, 30), (Z, Z, P, P, F, F), False), ((32, 900, 1), (F, F, Z, Z, P, P), False)]
 MARCHING = [((118, 112, 101), (P, P, P, P, Z, F), True), ((121, 115, 98), PLUME, True), ((128, 112, 90), PLUME, False),
             ((700, 50, 40), PLUME, True)]
 
@@ -116,7 +120,10 @@ def masked_system(cfg, prob, mask, anchor, rhs):
     return apply, np.where(active, rhs.astype(np.float64) + fixed.ravel(), 0.0), active
 
 
-@pytest.mark.parametrize("res,modes,ball", RESIDENT + MARCHING, ids=["x".join(map(str, r)) + ("-solid" if b else "") for r, _, b in RESIDENT + MARCHING])
+FORMS = RESIDENT + WRAPPED + MARCHING
+
+
+@pytest.mark.parametrize("res,modes,ball", FORMS, ids=["x".join(map(str, r)) + ("-solid" if b else "") for r, _, b in FORMS])
 def test_solutions_satisfy_the_system(cuda, res, modes, ball):
     cfg, prob, mask, rhs = problem(res, modes, ball)
     n = int(np.prod(res))
