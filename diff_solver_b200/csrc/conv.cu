@@ -80,14 +80,19 @@ bool make_weight_map(CUtensorMap* map, const void* base, uint32_t rows, uint32_t
 // ------------------------------------------------------------------ forward
 constexpr int kConvThreads = 128;
 
-template <int CIN, int COUT>
+// Bytes of a CTA's stages: two CTAs per SM, or four.  Deep stages keep the
+// MMAs of few CTAs fed, many CTAs do that for one another
+// (launch_conv_forward has both sides).
+constexpr uint32_t kDeepStages = 98304u, kShallowStages = 49152u;
+
+template <int CIN, int COUT, uint32_t BUDGET>
 struct ConvSmem {
     static constexpr uint32_t a_bytes = 128u * CIN * 2u;
     static constexpr uint32_t b_bytes_raw = static_cast<uint32_t>(COUT) * CIN * 2u;
     static constexpr uint32_t b_bytes = (b_bytes_raw + 1023u) / 1024u * 1024u;
     static constexpr uint32_t stage_bytes = a_bytes + b_bytes;
-    // loads in flight: what 96 KB hold, so that two CTAs fit an SM
-    static constexpr int stages = 98304u / stage_bytes < 12u ? static_cast<int>(98304u / stage_bytes) : 12;
+    static constexpr uint32_t fit = BUDGET / stage_bytes;
+    static constexpr int stages = fit < 3u ? 3 : (fit < 12u ? static_cast<int>(fit) : 12);
     static constexpr uint32_t total = 1024u /*alignment slack*/ + stages * stage_bytes + 256u /*barriers*/;
     static constexpr uint32_t tmem_cols = COUT <= 32 ? 32u : 64u;
 };
@@ -102,10 +107,10 @@ struct ConvArgs {
 };
 
 // One CTA = one tile of 128 output voxels (a bx * by * bz box of one batch).
-template <int CIN, int COUT>
+template <int CIN, int COUT, uint32_t BUDGET>
 __global__ void __launch_bounds__(kConvThreads) conv3_forward_kernel(const __grid_constant__ CUtensorMap act_map,
                                                                      const __grid_constant__ CUtensorMap w_map, ConvArgs a) {
-    using L = ConvSmem<CIN, COUT>;
+    using L = ConvSmem<CIN, COUT, BUDGET>;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~uintptr_t(1023u));
     unsigned char* a_tiles = smem;
@@ -437,6 +442,16 @@ XsStatus launch_conv_slab(cudaStream_t st, const VolumeShape& s, const SlabPlan&
     return check_launch();
 }
 
+template <int CIN, int COUT, uint32_t BUDGET>
+XsStatus launch_conv_boxes(cudaStream_t st, const CUtensorMap& am, const CUtensorMap& wm, const ConvArgs& args, uint64_t tiles) {
+    using L = ConvSmem<CIN, COUT, BUDGET>;
+    static DeviceOnce configured;
+    if (!configured.run([] { return cudaFuncSetAttribute(conv3_forward_kernel<CIN, COUT, BUDGET>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total); }))
+        return XS_CUDA_ERROR;
+    conv3_forward_kernel<CIN, COUT, BUDGET><<<static_cast<unsigned>(tiles), kConvThreads, L::total, st>>>(am, wm, args);
+    return check_launch();
+}
+
 template <int CIN, int COUT>
 XsStatus launch_conv_forward(cudaStream_t st, const VolumeShape& s, const __nv_bfloat16* in, const __nv_bfloat16* w, const float* bias,
                              __nv_bfloat16* out, bool relu, int* error) {
@@ -448,7 +463,7 @@ XsStatus launch_conv_forward(cudaStream_t st, const VolumeShape& s, const __nv_b
     // has too few MMAs behind one box to wait for (16 -> 32 at 32^3 14.1 us
     // against 11.1; by both slopes they meet near 100,000 voxels), and from 32
     // channels on a box fills an MMA's time anyway (32 -> 16 at 8 x 32^3 52.0
-    // against 51.3, 64 -> 64 at 16^3 16.2 against 9.9).
+    // against 39.1, 64 -> 64 at 16^3 16.2 against 9.9).
     if constexpr (CIN == 16) {
         SlabPlan plan;
         if (static_cast<uint64_t>(s.x) * s.y * s.z * s.batch >= kSlabMinVoxels && slab_plan<CIN, COUT>(s, plan))
@@ -456,14 +471,20 @@ XsStatus launch_conv_forward(cudaStream_t st, const VolumeShape& s, const __nv_b
     }
     CUtensorMap am, wm;
     if (!make_activation_map(&am, in, s, CIN, bx, by, bz) || !make_weight_map(&wm, w, COUT, CIN)) return XS_CUDA_ERROR;
-    using L = ConvSmem<CIN, COUT>;
-    static DeviceOnce configured;
-    if (!configured.run([] { return cudaFuncSetAttribute(conv3_forward_kernel<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::total); }))
-        return XS_CUDA_ERROR;
-    ConvArgs args{s, bx, by, bz, bias, out, relu ? 1 : 0, error};
+    const ConvArgs args{s, bx, by, bz, bias, out, relu ? 1 : 0, error};
     const uint64_t tiles = static_cast<uint64_t>(s.batch) * (s.z / bz) * (s.y / by) * (s.x / bx);
-    conv3_forward_kernel<CIN, COUT><<<static_cast<unsigned>(tiles), kConvThreads, L::total, st>>>(am, wm, args);
-    return check_launch();
+    // Few tiles: deep stages, 64 -> 64 with 128 tiles 10.5 us (shallow 12.5), 16 ->
+    // 64 with 512 22.9 (27.0).  Many: shallow ones and twice the CTAs, with 2,048
+    // tiles 32 -> 16 39.1 (deep 51.2), 32 -> 32 47.4 (55.5), 64 -> 16 56.3 (63.4), 64
+    // -> 64 76.3 (78.2), with 12,284 32 -> 16 196 (277).  They meet between 512 and
+    // 1,024 tiles; before that where a tile's products are few, 32 channels to at
+    // most 32 (456 tiles, 32 -> 16 14.5, deep 16.5; 32 -> 32 17.3, deep 18.6), and
+    // where its box is many short rows, x of 2 or 4 (340 to 426 tiles, 64 -> 32 14.6
+    // to 16.5, deep 16.7 to 18.7; 160, 64 -> 32 12.4, deep 10.6).
+    const bool early = (CIN == 32 && COUT <= 32) || s.x < 8u;
+    const uint64_t few = 148u * (early ? 2u : 4u);
+    return tiles <= few ? launch_conv_boxes<CIN, COUT, kDeepStages>(st, am, wm, args, tiles)
+                        : launch_conv_boxes<CIN, COUT, kShallowStages>(st, am, wm, args, tiles);
 }
 
 // The 128-voxel output tile: as wide in x as the volume allows (up to 128),
@@ -561,7 +582,8 @@ template <int CIN, int COUT>
 __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_constant__ CUtensorMap x_map,
                                                                    const __grid_constant__ CUtensorMap dy_map, WgradArgs a) {
     constexpr uint32_t count = 27u * CIN * COUT;
-    if (a.redo) {
+    constexpr bool kAfterSlabs = CIN <= 32 && COUT <= 32;
+    if constexpr (kAfterSlabs) if (a.redo) {
         // the sums are formed while the flags are on their way; a CTA per SM
         // (more do not fit beside the boxes' memory)
         constexpr int kSums = (count + kWgradCtas * kConvThreads - 1u) / (kWgradCtas * kConvThreads);
@@ -689,18 +711,20 @@ __global__ void __launch_bounds__(kConvThreads) conv3_wgrad_kernel(const __grid_
     tc::tc_fence_before();
     __syncthreads();
     if (warp == 0) tc::tmem_dealloc(tmem, 256);
-    if (!a.redo) return;
-    __shared__ uint32_t before;
-    __threadfence();  // the CTA's sums before its ticket
-    __syncthreads();
-    if (threadIdx.x == 0) before = atomicAdd(a.ticket, 1u);
-    __syncthreads();
-    if (before != gridDim.x * gridDim.y - 1u) return;
-    __threadfence();
-    PartialSums<1> sums;
-    for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) {
-        sums.form(a.partial, nctas, count, i, 0u);
-        sums.add_to(a.dw, a.accumulate, count, i, 0u);
+    if constexpr (kAfterSlabs) {
+        if (!a.redo) return;
+        __shared__ uint32_t before;
+        __threadfence();  // the CTA's sums before its ticket
+        __syncthreads();
+        if (threadIdx.x == 0) before = atomicAdd(a.ticket, 1u);
+        __syncthreads();
+        if (before != gridDim.x * gridDim.y - 1u) return;
+        __threadfence();
+        PartialSums<1> sums;
+        for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) {
+            sums.form(a.partial, nctas, count, i, 0u);
+            sums.add_to(a.dw, a.accumulate, count, i, 0u);
+        }
     }
 }
 
@@ -902,9 +926,9 @@ bool wgrad_slab_plan(const VolumeShape& s, uint32_t ctas, WslabArgs& best) {
 __global__ void wgrad_reduce_kernel(const float* __restrict__ partial, uint32_t ctas, uint32_t count, float* __restrict__ dw, int accumulate) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
-    PartialSums<1> sums;
-    sums.form(partial, ctas, count, i, 0u);
-    sums.add_to(dw, accumulate, count, i, 0u);
+    float acc = 0.0f;
+    for (uint32_t c = 0; c < ctas; ++c) acc += partial[static_cast<size_t>(c) * count + i];
+    dw[i] = accumulate ? dw[i] + acc : acc;
 }
 
 uint32_t wgrad_ctas(const VolumeShape& s) {

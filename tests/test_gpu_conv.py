@@ -133,6 +133,27 @@ def test_conv_from_halo_slabs(cuda, cout, shape, batch):
         assert bool(((one.float() - out.float()).abs() <= 2.0 ** -7 * one.float().abs() + 1e-4).all())
 
 
+@pytest.mark.parametrize("cin,cout,shape,batch", [(32, 16, (32, 32, 37), 1), (32, 32, (32, 32, 38), 1), (32, 64, (64, 64, 19), 1), (16, 64, (32, 32, 74), 1),
+                                                  (64, 16, (32, 64, 38), 1), (64, 32, (64, 36, 33), 1), (64, 64, (128, 37, 17), 1), (32, 16, (64, 64, 33), 2)])
+def test_conv_on_either_side_of_the_deep_stages(cuda, cin, cout, shape, batch):
+    """Numbers of 128-voxel tiles at, just past and well past those that take
+    deep stages (296 and 592), as many CTAs as an SM holds and more."""
+    import torch
+    from diff_solver_b200 import _native as N
+    nx, ny, nz = shape
+    g = torch.Generator(device="cuda").manual_seed(cin + cout)
+    x = torch.randn(batch, nz, ny, nx, cin, generator=g, device="cuda").to(torch.bfloat16)
+    w = (torch.randn(27, cout, cin, generator=g, device="cuda") / (27 * cin) ** 0.5).to(torch.bfloat16)
+    out = torch.full((batch, nz, ny, nx, cout), float("nan"), dtype=torch.bfloat16, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    N.check("conv", N.lib().xs_conv3d_bf16(None, batch, nx, ny, nz, cin, cout, x.data_ptr(), w.data_ptr(), None, out.data_ptr(), 0, err.data_ptr()))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    want = reference_conv(x.double(), w.double(), None, False)
+    # exact products, FP32 sums of 27 cin of them, one rounding to BF16
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 27 * cin * 2.0 ** -24).all())
+
+
 @pytest.mark.parametrize("cin,cout,shape,batch", [(16, 16, (32, 32, 32), 1), (16, 32, (64, 30, 18), 1), (32, 32, (16, 24, 50), 2),
                                                   (16, 16, (8, 16, 30), 8), (16, 16, (16, 16, 8), 2)])
 @pytest.mark.parametrize("value", [float("inf"), float("nan")], ids=["inf", "nan"])
